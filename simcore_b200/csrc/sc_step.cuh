@@ -131,31 +131,56 @@ __device__ __forceinline__ void bond_pair_sum(const DevState &d, int b, int e0, 
   F[0] = F[1] = F[2] = 0.0;
   T[0] = T[1] = T[2] = 0.0;
   if (d.nx) bond_xlink_sum<ND>(d, b, F, T);
+  // Slots are loaded in batches whose loads are all in flight together, then
+  // added in order: bound by the round trips to L2, one after another in a
+  // plain loop's remainder, and most bonds have one to five slots.  20,000
+  // filaments of 5 to 200 bonds, 20 mixed steps: 9.45 ms before, 8.97 ms now.
   if (PREC == 0) {
+    constexpr int BATCH = 3;
     const double2 *c = reinterpret_cast<const double2 *>(d.cf64) + 4 * (size_t)e0;
-#pragma unroll 2
-    for (int e = e0; e < e1; ++e, c += 4) {
-      const double2 v0 = c[0], v1 = c[1], v2 = c[2];
-      F[0] += v0.x;
-      F[1] += v0.y;
-      if (ND == 3) F[2] += v1.x;
-      T[0] += v1.y;
-      T[1] += v2.x;
-      T[2] += v2.y;
+    for (int e = e0; e < e1; e += BATCH, c += 4 * BATCH) {
+      double2 v[BATCH][3];
+#pragma unroll
+      for (int q = 0; q < BATCH; ++q)
+        if (e + q < e1) {
+          v[q][0] = c[4 * q];
+          v[q][1] = c[4 * q + 1];
+          v[q][2] = c[4 * q + 2];
+        }
+#pragma unroll
+      for (int q = 0; q < BATCH; ++q)
+        if (e + q < e1) {
+          F[0] += v[q][0].x;
+          F[1] += v[q][0].y;
+          if (ND == 3) F[2] += v[q][1].x;
+          T[0] += v[q][1].y;
+          T[1] += v[q][2].x;
+          T[2] += v[q][2].y;
+        }
     }
   } else {
+    constexpr int BATCH = 4;
     float sF[3] = {0.f, 0.f, 0.f}, cF[3] = {0.f, 0.f, 0.f};
     float sT[3] = {0.f, 0.f, 0.f}, cT[3] = {0.f, 0.f, 0.f};
     const float4 *c = reinterpret_cast<const float4 *>(d.cf32) + 2 * (size_t)e0;
-#pragma unroll 4
-    for (int e = e0; e < e1; ++e, c += 2) {
-      const float4 v0 = c[0], v1 = c[1];
-      kahan_add(sF[0], cF[0], v0.x);
-      kahan_add(sF[1], cF[1], v0.y);
-      if (ND == 3) kahan_add(sF[2], cF[2], v0.z);
-      kahan_add(sT[0], cT[0], v0.w);
-      kahan_add(sT[1], cT[1], v1.x);
-      kahan_add(sT[2], cT[2], v1.y);
+    for (int e = e0; e < e1; e += BATCH, c += 2 * BATCH) {
+      float4 v[BATCH][2];
+#pragma unroll
+      for (int q = 0; q < BATCH; ++q)
+        if (e + q < e1) {
+          v[q][0] = c[2 * q];
+          v[q][1] = c[2 * q + 1];
+        }
+#pragma unroll
+      for (int q = 0; q < BATCH; ++q)
+        if (e + q < e1) {
+          kahan_add(sF[0], cF[0], v[q][0].x);
+          kahan_add(sF[1], cF[1], v[q][0].y);
+          if (ND == 3) kahan_add(sF[2], cF[2], v[q][0].z);
+          kahan_add(sT[0], cT[0], v[q][0].w);
+          kahan_add(sT[1], cT[1], v[q][1].x);
+          kahan_add(sT[2], cT[2], v[q][1].y);
+        }
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
