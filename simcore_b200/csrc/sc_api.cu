@@ -365,61 +365,93 @@ sc_status maybe_rebuild(sc_ctx *c) {
   return rebuild(c);
 }
 
-// Integrator work units over the filaments in order: runs of whole
-// filaments of at most warp_sites sites each go to the warp-synchronous
-// kernel (one lane per site, at most 32 sites per group); longer filaments go
-// to the block kernel (runs of whole filaments up to C sites per block).
+// Integrator work units over the filaments in order: runs of whole filaments
+// of at most warp_sites sites each go to the team kernel (one warp, K sites a
+// lane), longer ones to the block kernel (runs of whole filaments up to C
+// sites per block).
 sc_status layout_integrator(sc_ctx *c) {
   const std::vector<int> &off = c->site_off;
   const int n = c->nf;
-  std::vector<int> blk_site0, blk_f0, blk_nf, blk_ns, wg_site0, wg_f0, wg_ns;
   int max_long = 0;
-  auto short_fil = [&](int f) { return off[f + 1] - off[f] <= c->warp_sites; };
-  for (int f = 0; f < n; ++f)
-    if (!short_fil(f)) max_long = std::max(max_long, off[f + 1] - off[f]);
+  for (int f = 0; f < n; ++f) {
+    const int nn = off[f + 1] - off[f];
+    if (nn > c->warp_sites) max_long = std::max(max_long, nn);
+  }
   c->C = c->block_sites > 0 ? c->block_sites
                             : (max_long <= 128 ? 128 : max_long <= 256 ? 256 : 512);
   if (max_long > c->C)
     return fail(c, SC_ERR_INVALID_ARG, "a %d-site filament does not fit %d-site blocks", max_long,
                 c->C);
+  const int team_max = c->warp_sites;
+  auto sites = [&](int f) { return off[f + 1] - off[f]; };
   // A work unit never mixes systems (its displacement maximum is one
   // system's).
   auto same = [&](int f, int f0) { return c->fil_rep.empty() || c->fil_rep[f] == c->fil_rep[f0]; };
+  auto team_end = [&](int f0, int k) {  // past the filaments of the team warp that starts at f0
+    int f = f0, used = 0;
+    while (f < n && sites(f) <= team_max && same(f, f0) && used + (sites(f) + k - 1) / k <= 32)
+      used += (sites(f++) + k - 1) / k;
+    return f;
+  };
+  // Sites per lane.  One is the shorter chain (100 x 21 sites, FP64: 12.8 us a
+  // step against 19.1 with two), two fill the warps better (15,839 x 17
+  // sites, FP64: 47.7 us against 73.7, with 5,280 warps instead of 15,839);
+  // a pass over the chip takes about 1.6 times as long with two, at 16 warps
+  // an SM instead of 20, so two pay where they save more than half the warps
+  // (the margin covers 20,000 filaments of 5 to 32 sites, 1.9 times fewer:
+  // 35 us with one, 50 with two) and one lane a site fills the chip at all.
+  long long warps[3] = {0, 0, 0};
+  for (int k = 1; k <= 2; ++k)
+    for (int f = 0; f < n;) {
+      if (sites(f) <= team_max) {
+        f = team_end(f, k);
+        ++warps[k];
+      } else {
+        ++f;
+      }
+    }
+  const int K = warps[1] > 148 * 20 && 4 * warps[1] >= 9 * warps[2] ? 2 : 1;
+  std::vector<int> blk_site0, blk_f0, blk_nf, blk_ns;
+  std::vector<int4> lanes;
+  bool uni = n > 0 && sites(0) <= team_max;
+  for (int f = 1; uni && f < n; ++f) uni = sites(f) == sites(0) && same(f, 0);
   int f = 0;
-  while (f < n) {
+  while (f < n && !uni) {
     const int s0 = off[f], f0 = f;
-    if (short_fil(f)) {
-      while (f < n && short_fil(f) && same(f, f0) && off[f + 1] - s0 <= 32) ++f;
-      wg_site0.push_back(s0);
-      wg_f0.push_back(f0);
-      wg_ns.push_back(off[f] - s0);
+    if (sites(f) <= team_max) {
+      f = team_end(f0, K);
+      const size_t base = lanes.size();
+      for (int q = f0; q < f; ++q)
+        for (int j = 0; j < sites(q); j += K)
+          lanes.push_back(make_int4(off[q] + j, q, j | sites(q) << 16, (q - f0) | (f - f0) << 8));
+      // Idle lanes name the warp's first site, of a filament without sites.
+      while (lanes.size() < base + 32) lanes.push_back(make_int4(s0, f0, 0, (f - f0) << 8));
     } else {
-      while (f < n && !short_fil(f) && same(f, f0) && off[f + 1] - s0 <= c->C) ++f;
+      while (f < n && sites(f) > team_max && same(f, f0) && off[f + 1] - s0 <= c->C) ++f;
       blk_site0.push_back(s0);
       blk_f0.push_back(f0);
       blk_nf.push_back(f - f0);
       blk_ns.push_back(off[f] - s0);
     }
   }
-  for (const int *q : {c->d.blk_site0, c->d.blk_f0, c->d.blk_nf, c->d.blk_ns, c->d.wg_site0,
-                       c->d.wg_f0, c->d.wg_ns})
-    dfree(c, const_cast<int *>(q));
-  auto up = [&](const int **dst, const std::vector<int> &v) -> sc_status {
-    int *q = nullptr;
+  DevState &d = c->d;
+  for (const void *q : {(const void *)d.blk_site0, (const void *)d.blk_f0, (const void *)d.blk_nf,
+                        (const void *)d.blk_ns, (const void *)d.tm_lane})
+    dfree(c, const_cast<void *>(q));
+  auto up = [&](auto **dst, const auto &v) -> sc_status {
+    using T = typename std::remove_reference<decltype(v)>::type::value_type;
+    T *q = nullptr;
     CKS(dalloc(c, &q, v.size()));
     if (!v.empty())
-      CK(cudaMemcpyAsync(q, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, c->st));
+      CK(cudaMemcpyAsync(q, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c->st));
     *dst = q;
     return SC_OK;
   };
-  DevState &d = c->d;
   CKS(up(&d.blk_site0, blk_site0));
   CKS(up(&d.blk_f0, blk_f0));
   CKS(up(&d.blk_nf, blk_nf));
   CKS(up(&d.blk_ns, blk_ns));
-  CKS(up(&d.wg_site0, wg_site0));
-  CKS(up(&d.wg_f0, wg_f0));
-  CKS(up(&d.wg_ns, wg_ns));
+  CKS(up(&d.tm_lane, lanes));
   CK(cudaStreamSynchronize(c->st));
   c->nblocks = (int)blk_f0.size();
   d.blk_maxf = 0;
@@ -429,19 +461,27 @@ sc_status layout_integrator(sc_ctx *c) {
   d.blk_uni_n = d.blk_uni_fpb = 0;
   if (!blk_f0.empty() && n > 0) {
     const int nn = off[1] - off[0], fpb = blk_nf[0];
-    bool uni = nn > 0 && fpb > 0 && (long long)blk_f0.size() == ((long long)n + fpb - 1) / fpb;
-    for (int q = 0; uni && q <= n; ++q) uni = off[q] == (long long)q * nn;
-    for (size_t i = 0; uni && i < blk_f0.size(); ++i) {
+    bool buni = nn > 0 && fpb > 0 && (long long)blk_f0.size() == ((long long)n + fpb - 1) / fpb;
+    for (int q = 0; buni && q <= n; ++q) buni = off[q] == (long long)q * nn;
+    for (size_t i = 0; buni && i < blk_f0.size(); ++i) {
       const long long f0 = (long long)i * fpb;
-      uni = blk_f0[i] == f0 && blk_nf[i] == std::min<long long>(fpb, n - f0) &&
-            blk_site0[i] == f0 * nn && blk_ns[i] == (long long)blk_nf[i] * nn;
+      buni = blk_f0[i] == f0 && blk_nf[i] == std::min<long long>(fpb, n - f0) &&
+             blk_site0[i] == f0 * nn && blk_ns[i] == (long long)blk_nf[i] * nn;
     }
-    if (uni) {
+    if (buni) {
       d.blk_uni_n = nn;
       d.blk_uni_fpb = fpb;
     }
   }
-  d.n_wg = (int)wg_f0.size();
+  d.n_tm = (int)(lanes.size() / 32);
+  d.tm_k = K;
+  d.tm_uni_n = d.tm_uni_lanes = d.tm_uni_fpw = 0;
+  if (uni) {
+    d.tm_uni_n = sites(0);
+    d.tm_uni_lanes = (sites(0) + K - 1) / K;
+    d.tm_uni_fpw = 32 / d.tm_uni_lanes;
+    d.n_tm = (n + d.tm_uni_fpw - 1) / d.tm_uni_fpw;
+  }
   sc::prepare_integrate(c->C);
   drop_graph(c);
   return SC_OK;
@@ -790,6 +830,7 @@ static sc_status add_systems(sc_ctx *c, int nrep, const double *radius, const ui
     q.linv = 1.0 / q.l;
     q.kappa = p[f].persistence_length;
     q.l2 = q.l * q.l;
+    q.l2inv = 1.0 / q.l2;
     double logLD = std::log(len[f] / p[f].diameter);
     double gperp = 4.0 * len[f] / (3.0 * nsf * logLD);
     double gpar = gperp / p[f].friction_ratio;

@@ -104,19 +104,23 @@ struct ReplicaConst {
   int p0, pcap;       // pair segment [p0, p0 + pcap), slots [2 p0, 2 (p0 + pcap))
 };
 
+// Rows of the longest system (bonds of the longest filament) above which the
+// fast 256- and 512-site integrator blocks solve by pcr_block instead of
+// Thomas lanes.
+constexpr int kPcrMinRows = 32;
+
 // Per-filament constants of the integrator.  The reciprocals are the
 // reference's own quotients (1.0 / friction_par_, 2.0 / friction_perp_, ...,
 // src/filament.cpp:783-830, 992-996), evaluated once on the host with the
 // same IEEE operations, so every use sees the bits the reference computes
 // inline.  112 bytes.
 struct FilConst {
-  double l, linv, kappa, l2;                   // bond length, 1/l, lp, l*l
+  double l, linv, kappa, l2, l2inv;            // bond length, 1/l, lp, l*l, 1/(l*l)
   double igpar, igperp, two_igperp, m1_igperp; // 1/g_par, 1/g_perp, 2/g_perp, -1/g_perp
   double dgam;                                 // 1/g_par - 1/g_perp
   double spar, sperp;                          // sqrt(24 g / delta)
   int site0, n;                                // first site, number of sites
   int rep, f_local;                            // system, index within it (noise key)
-  int pad0, pad1;
 };
 
 // Launch-invariant device pointers of one context.
@@ -145,12 +149,15 @@ struct DevState {
   // but the last full, sites numbered filament by filament from 0: blocks
   // and sites then find their filaments by arithmetic (0: read the tables).
   int blk_uni_n, blk_uni_fpb;
-  // integrator warp groups (filaments of at most 32 sites): runs of whole
-  // filaments, one lane per site
-  int n_wg;
-  const int *wg_site0;     // per group: first site
-  const int *wg_f0;        // per group: first filament
-  const int *wg_ns;        // per group: site count
+  // integrator teams (filaments of at most 32 sites): warps of
+  // whole filaments, ceil(n / K) lanes each
+  int n_tm;                // warps
+  int tm_k;                // sites per lane
+  const int4 *tm_lane;     // 32 per warp: the lane's first site; its filament; its first site's
+                           // index | filament sites << 16; filament in the warp | warp's filaments << 8
+  // Equal filaments of tm_uni_n sites, tm_uni_lanes lanes each, tm_uni_fpw to
+  // a warp: lanes find their sites by arithmetic (0: read the table).
+  int tm_uni_n, tm_uni_lanes, tm_uni_fpw;
   // sites (SoA, 3 components each)
   double *r[3], *rp[3], *fr[3], *dz[3];
   double *dt;

@@ -161,7 +161,7 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
       // step's too), per rebuild the captured sequence.  A step is its pair
       // kernel (unless fused; near-parallel pairs are evaluated in place),
       // thermo and one or two integrator kernels.
-      const int int_l = (c->d.n_wg > 0 ? 1 : 0) + (c->nblocks > 0 ? 1 : 0);
+      const int int_l = (c->d.n_tm > 0 ? 1 : 0) + (c->nblocks > 0 ? 1 : 0);
       const long long per_bd =
           c->desc.interaction_flag
               ? 1 + (c->d.nx ? 2 : 0) +

@@ -26,7 +26,7 @@
 #include "sc_cells.cuh"
 #include "sc_pair.cuh"
 #include "sc_step.cuh"
-#include "sc_step_warp.cuh"
+#include "sc_step_team.cuh"
 
 namespace sc {
 
@@ -1635,17 +1635,20 @@ int launch_integrate(const SysConst &k, const DevState &d, int nblocks, int C,
     return launch_integrate_fast(k, d, nblocks, C, midstep, rbuf, interaction, capture, st,
                                  fuse && interaction);
   int launched = 0;
-  if (d.n_wg > 0) {
-    const int grid = cdiv(d.n_wg, kIntWarps);
-#define SC_INTEGRATE_WARP(ND, P)                                              \
-  launch_pdl(k_integrate_warp<ND, P, false>, dim3(grid), dim3(kIntWarps * 32), 0, st, k, d, midstep, rbuf, \
-                                                                  interaction, capture)
+  if (d.n_tm > 0) {
+    const int grid = cdiv(d.n_tm, kTeamWarps);
+#define SC_INTEGRATE_TEAM(ND, P)                                                           \
+  ((d.tm_k == 1)                                                                           \
+       ? launch_pdl(k_integrate_team<ND, P, false, 1>, dim3(grid), dim3(kTeamWarps * 32),  \
+                    team_smem_bytes(1), st, k, d, midstep, rbuf, interaction, capture)     \
+       : launch_pdl(k_integrate_team<ND, P, false, 2>, dim3(grid), dim3(kTeamWarps * 32),  \
+                    team_smem_bytes(2), st, k, d, midstep, rbuf, interaction, capture))
     if (k.n_dim == 3) {
-      if (prec == 0) SC_INTEGRATE_WARP(3, 0); else SC_INTEGRATE_WARP(3, 1);
+      if (prec == 0) SC_INTEGRATE_TEAM(3, 0); else SC_INTEGRATE_TEAM(3, 1);
     } else {
-      if (prec == 0) SC_INTEGRATE_WARP(2, 0); else SC_INTEGRATE_WARP(2, 1);
+      if (prec == 0) SC_INTEGRATE_TEAM(2, 0); else SC_INTEGRATE_TEAM(2, 1);
     }
-#undef SC_INTEGRATE_WARP
+#undef SC_INTEGRATE_TEAM
     ++launched;
   }
   if (nblocks == 0) return launched;

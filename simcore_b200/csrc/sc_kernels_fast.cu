@@ -10,7 +10,7 @@
 #include "sc_launch.h"
 #include "sc_pair.cuh"
 #include "sc_step.cuh"
-#include "sc_step_warp.cuh"
+#include "sc_step_team.cuh"
 
 namespace sc {
 
@@ -60,10 +60,14 @@ template <int ND, bool FUSE>
 static int launch_fast(const SysConst &k, const DevState &d, int nblocks, int C, int midstep,
                        int rbuf, int interaction, int capture, cudaStream_t st) {
   int launched = 0;
-  if (d.n_wg > 0) {
-    const int grid = (d.n_wg + kIntWarps - 1) / kIntWarps;
-    launch_pdl(k_integrate_warp<ND, 1, true, FUSE>, dim3(grid), dim3(kIntWarps * 32), 0, st, k, d, midstep, rbuf,
-                                                                        interaction, capture);
+  if (d.n_tm > 0) {
+    const int grid = (d.n_tm + kTeamWarps - 1) / kTeamWarps;
+    if (d.tm_k == 1)
+      launch_pdl(k_integrate_team<ND, 1, true, 1, FUSE>, dim3(grid), dim3(kTeamWarps * 32),
+                 team_smem_bytes(1), st, k, d, midstep, rbuf, interaction, capture);
+    else
+      launch_pdl(k_integrate_team<ND, 1, true, 2, FUSE>, dim3(grid), dim3(kTeamWarps * 32),
+                 team_smem_bytes(2), st, k, d, midstep, rbuf, interaction, capture);
     ++launched;
   }
   if (nblocks == 0) return launched;

@@ -82,6 +82,54 @@ __device__ __forceinline__ void store_geom(const DevState &d, int buf, int b,
   }
 }
 
+// IEEE division (round to nearest) by a shared reciprocal, for the exact
+// integrator: several quotients have one divisor, and a quotient's chain is
+// the integrator's critical path.  y = RN(1/b) from the hardware's approximate
+// reciprocal by one third-order step, which leaves it within one ulp, and
+// Markstein's correction y + y (1 - b y), whose result is the correctly
+// rounded reciprocal unless b's significand is all ones (Markstein, IBM J.
+// Res. Dev. 34:111-119, 1990; Muller et al., Handbook of Floating-Point
+// Arithmetic, 2nd ed., sec. 4.7).  A quotient starts as q0 = x y, within two
+// ulps of x/b; one correction q1 = q0 + y (x - b q0) makes it faithful, and a
+// second one on a faithful quotient is correctly rounded (the same theorem:
+// x - b q1 is exact); a zero x keeps q0, a zero of the quotient's sign.  The
+// result has the bits of x / b where `ok` holds at the end: every exponent
+// leaves room for the intermediates, and no divisor's significand is all ones.
+// The caller repeats its work with the compiler's division where it does not,
+// so that no quotient pays for a branch.  Measured, one warp: 126 cycles for
+// the compiler's division (two independent ones do not overlap: 262); here 61
+// for y and 47 for each quotient, which do.
+__device__ __forceinline__ bool mid_exponent(double x) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  return e - (1023u - 450u) < 900u;
+}
+__device__ __forceinline__ double recip_rn(double b, bool &ok) {
+  const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+  ok = ok && mid_exponent(b) && !(lo == 0xffffffffu && (hi & 0xfffffu) == 0xfffffu);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  double e = __fma_rn(-b, y, 1.0);
+  y = __fma_rn(y, __fma_rn(e, e, e), y);
+  e = __fma_rn(-b, y, 1.0);
+  return __fma_rn(e, y, y);
+}
+__device__ __forceinline__ double div_rn(double x, double b, double y, bool &ok) {
+  const bool zero = x == 0.0;
+  ok = ok && (mid_exponent(x) || zero);
+  const double q0 = __dmul_rn(x, y);
+  const double q1 = __fma_rn(__fma_rn(-b, q0, x), y, q0);
+  const double q2 = __fma_rn(__fma_rn(-b, q1, x), y, q1);
+  return zero ? q0 : q2;
+}
+// One quotient by a divisor whose RN(1/b) is at hand.
+__device__ __forceinline__ double div_by(double x, double b, double y) {
+  bool ok = mid_exponent(b);
+  const double q = div_rn(x, b, y, ok);
+  if (ok) return q;
+  asm volatile("" : "+d"(x));  // a branch: not computed beside the fast path
+  return x / b;
+}
+
 __device__ __forceinline__ void cross3(const double *a, const double *b,
                                        double *c) {
   c[0] = a[1] * b[2] - a[2] * b[1];
@@ -252,32 +300,154 @@ __device__ __forceinline__ void bond_pair_eval_sum(const SysConst &k, const DevS
 // filament lf of the block, lane C/2 + lf for the backward determinant), so
 // a block's serial work occupies one or two warps instead of every warp.
 
-// Thomas algorithm of the reference's tridiagonal_solver
-// (src/linear_algebra.cpp:164-197); n unknowns, in place.  The previous
-// row's c and d stay in registers (same values, same operations as reading
-// them back).
-__device__ __forceinline__ void thomas(double *a, const double *b, double *c,
-                                       double *d, int n) {
-  n--;
-  double cp = c[0] / b[0];
-  double dp = d[0] / b[0];
-  c[0] = cp;
-  d[0] = dp;
-  for (int i = 1; i < n; ++i) {
-    const double am = a[i - 1], bi = b[i];
-    const double cn = c[i] / (bi - am * cp);
-    const double dn = (d[i] - am * dp) / (bi - am * cp);
-    c[i] = cn;
-    d[i] = dn;
-    cp = cn;
-    dp = dn;
+// The reference's tridiagonal_solver (Thomas, src/linear_algebra.cpp:164-197)
+// in two parts, its operations in its order, so its bits: the elimination of
+// the matrix (den_i = b_i - a_{i-1} c'_{i-1}, c'_i = c_i / den_i) and the
+// elimination and back substitution of a right-hand side (d'_i = (d_i -
+// a_{i-1} d'_{i-1}) / den_i).  Split, the matrix part of every system and the
+// determinants run at once on different lanes, before the forces are known,
+// and a right-hand side's chain holds a quotient by a known reciprocal instead
+// of a division.  Bound by that serial chain: inside the integrator of 21-site
+// filaments 250 cycles a row for the matrices with the determinants and 145 a
+// right-hand side, where one solve with the compiler's division took 346 and
+// the determinants 85.  Operands are loaded a row ahead of the chain.  The
+// matrices are symmetric with couplings h (h_i couples rows i and i + 1; NEG:
+// -h_i); DIAG2: every diagonal element is 2.
+template <bool NEG, bool DIAG2>
+__device__ __forceinline__ void tridiag_factor_ieee(const double *h, const double *b, double *den,
+                                                    double *inv, double *up, int m) {
+  double cp = 0.0;
+  for (int i = 0; i < m; ++i) {
+    const double bi = DIAG2 ? 2.0 : b[i];
+    const double a = i > 0 ? (NEG ? -h[i - 1] : h[i - 1]) : 0.0;
+    const double dd = i > 0 ? bi - a * cp : bi;
+    den[i] = dd;
+    inv[i] = 1.0 / dd;
+    if (i < m - 1) up[i] = cp = (NEG ? -h[i] : h[i]) / dd;
   }
-  dp = (d[n] - a[n - 1] * dp) / (b[n] - a[n - 1] * cp);
-  d[n] = dp;
-  for (int i = n; i-- > 0;) {
-    dp = d[i] - c[i] * dp;
-    d[i] = dp;
+}
+// A shared-memory array named by its 32-bit address, for the routines below:
+// they are functions of their own, so that their loops keep their registers
+// (inlined into the integrators, at their register caps, a row took twice as
+// long), and take addresses that are known to be shared memory's.
+typedef unsigned sptr;
+__device__ __forceinline__ sptr to_sptr(const double *p) {
+  return (sptr)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ double *of_sptr(sptr a) {
+  return static_cast<double *>(__cvta_shared_to_generic(a));
+}
+
+template <bool NEG>
+static __device__ __noinline__ void tridiag_rhs_fn(sptr ah, sptr aden, sptr ainv, sptr aup, sptr ad,
+                                            sptr ax, int m) {
+  const double *h = of_sptr(ah), *den = of_sptr(aden), *inv = of_sptr(ainv), *up = of_sptr(aup);
+  const double *d = of_sptr(ad);
+  double *x = of_sptr(ax);
+  bool ok = true;
+  double v = div_rn(d[0], den[0], inv[0], ok);
+  x[0] = v;
+  double hn = h[0], dn = d[1], bn = den[1], yn = inv[1];
+  for (int i = 1; i < m; ++i) {
+    const double a = NEG ? -hn : hn, di = dn, bi = bn, yi = yn;
+    if (i + 1 < m) {
+      hn = h[i];
+      dn = d[i + 1];
+      bn = den[i + 1];
+      yn = inv[i + 1];
+    }
+    v = div_rn(di - a * v, bi, yi, ok);
+    x[i] = v;
   }
+  if (!ok) {
+    v = d[0] / den[0];
+    x[0] = v;
+    for (int i = 1; i < m; ++i) {
+      const double a = NEG ? -h[i - 1] : h[i - 1];
+      v = (d[i] - a * v) / den[i];
+      x[i] = v;
+    }
+  }
+  double cn = up[m - 2];
+  dn = x[m - 2];
+  for (int i = m - 2; i >= 0; --i) {
+    const double ci = cn, di = dn;
+    if (i > 0) {
+      cn = up[i - 1];
+      dn = x[i - 1];
+    }
+    v = di - ci * v;
+    x[i] = v;
+  }
+}
+
+template <bool NEG>
+__device__ __forceinline__ void tridiag_rhs(const double *h, const double *den, const double *inv,
+                                            const double *up, const double *d, double *x, int m) {
+  tridiag_rhs_fn<NEG>(to_sptr(h), to_sptr(den), to_sptr(inv), to_sptr(up), to_sptr(d), to_sptr(x),
+                      m);
+}
+
+// Two recurrences of one filament of n sites side by side on one lane, for
+// the exact step: the elimination of a matrix (mat: none without it) and a
+// metric determinant of CalculateBendingForces (src/filament.cpp:627-660) --
+// TRAIL: det_b from the head, to dt[n] .. dt[1]; else det_t from the tail, to
+// dt[0] .. dt[n - 1].  The projection matrix (2, -cos) goes with det_t, the
+// tension matrix with det_b, so lanes of both kinds run one instruction stream.
+static __device__ __noinline__ void factor_and_minors_fn(bool trail, bool mat, sptr acz, sptr aoff,
+                                                  sptr adiag, sptr aden, sptr ainv, sptr aup,
+                                                  sptr adt, int n) {
+  const double *cz = of_sptr(acz), *off = of_sptr(aoff), *diag = of_sptr(adiag);
+  double *den = of_sptr(aden), *inv = of_sptr(ainv), *up = of_sptr(aup), *dt = of_sptr(adt);
+  const int m = n - 1;  // rows
+  const double *h = trail ? off : cz;
+  const double sg = mat ? (trail ? 1.0 : -1.0) : 0.0;
+  double x0 = 1.0, x1 = 2.0;
+  dt[trail ? n : 0] = x0;
+  dt[trail ? n - 1 : 1] = x1;
+  double c = cz[trail ? n - 3 : 0];
+  double hi = sg * h[0], hn = m > 2 ? sg * h[1] : 0.0;
+  double bn = trail ? diag[1] : 2.0;
+  bool ok = true;
+  double dd = trail ? diag[0] : 2.0;
+  double y = recip_rn(dd, ok);
+  double cp = div_rn(hi, dd, y, ok);
+  if (mat) {
+    den[0] = dd;
+    inv[0] = y;
+    up[0] = cp;
+  }
+  for (int i = 1; i < m; ++i) {  // row i, minor i + 1
+    const double ai = hi, bi = bn, ci = hn;
+    hi = hn;
+    if (i + 1 < m) bn = trail ? diag[i + 1] : 2.0;
+    hn = i + 2 < m ? sg * h[i + 1] : 0.0;
+    const double cn = i + 2 < n ? cz[trail ? n - i - 3 : i] : 0.0;
+    const double x2 = 2 * x1 - c * c * x0;
+    dt[trail ? n - i - 1 : i + 1] = x2;
+    x0 = x1;
+    x1 = x2;
+    c = cn;
+    dd = bi - ai * cp;
+    y = recip_rn(dd, ok);
+    cp = div_rn(ci, dd, y, ok);
+    if (mat) {
+      den[i] = dd;
+      inv[i] = y;
+      up[i] = cp;
+    }
+  }
+  if (mat && !ok) {
+    if (trail) tridiag_factor_ieee<false, false>(off, diag, den, inv, up, m);
+    else tridiag_factor_ieee<true, true>(cz, nullptr, den, inv, up, m);
+  }
+}
+__device__ __forceinline__ void factor_and_minors(bool trail, bool mat, const double *cz,
+                                                  const double *off, const double *diag,
+                                                  double *den, double *inv, double *up,
+                                                  double *dt, int n) {
+  factor_and_minors_fn(trail, mat, to_sptr(cz), to_sptr(off), to_sptr(diag), to_sptr(den),
+                       to_sptr(inv), to_sptr(up), to_sptr(dt), n);
 }
 
 // 1/x for the fast integrator: from the hardware's FP64 approximate
@@ -336,38 +506,42 @@ __device__ __forceinline__ double recip_t(double x) { return recip_nr(x); }
 __device__ __forceinline__ float recip_t(float x) { return rcp_approx(x); }
 
 // FAST: one reciprocal per row instead of two divisions (FP64: recip_nr;
-// FP32: the approximate reciprocal, within an ulp).
+// FP32: the approximate reciprocal, within an ulp).  Each row's operands are
+// loaded a row ahead of the chain.
 template <class T>
 __device__ __forceinline__ void thomas_fast(T *a, const T *b, T *c, T *d, int n) {
   n--;
   T r = recip_t(b[0]);
   T cp = c[0] * r;
   T dp = d[0] * r;
+  T an = a[0], bn = b[1], cn = n > 1 ? c[1] : T(0), dn = d[1];
   c[0] = cp;
   d[0] = dp;
   for (int i = 1; i < n; ++i) {
-    const T am = a[i - 1];
-    r = recip_t(b[i] - am * cp);
-    const T cn = c[i] * r;
-    const T dn = (d[i] - am * dp) * r;
-    c[i] = cn;
-    d[i] = dn;
-    cp = cn;
-    dp = dn;
-  }
-  dp = (d[n] - a[n - 1] * dp) * recip_t(b[n] - a[n - 1] * cp);
-  d[n] = dp;
-  for (int i = n; i-- > 0;) {
-    dp = d[i] - c[i] * dp;
+    const T am = an, bi = bn, ci = cn, di = dn;
+    an = a[i];
+    bn = b[i + 1];
+    cn = i + 1 < n ? c[i + 1] : T(0);
+    dn = d[i + 1];
+    r = recip_t(bi - am * cp);
+    cp = ci * r;
+    dp = (di - am * dp) * r;
+    c[i] = cp;
     d[i] = dp;
   }
-}
-
-template <bool FAST>
-__device__ __forceinline__ void solve_tridiag(double *a, const double *b, double *c,
-                                              double *d, int n) {
-  if (FAST) thomas_fast(a, b, c, d, n);
-  else thomas(a, b, c, d, n);
+  dp = (dn - an * dp) * recip_t(bn - an * cp);
+  d[n] = dp;
+  cn = c[n - 1];
+  dn = d[n - 1];
+  for (int i = n - 1; i >= 0; --i) {
+    const T ci = cn, di = dn;
+    if (i > 0) {
+      cn = c[i - 1];
+      dn = d[i - 1];
+    }
+    dp = di - ci * dp;
+    d[i] = dp;
+  }
 }
 
 // Two-sided ("twisted") elimination of one tridiagonal system of n rows for
@@ -514,8 +688,18 @@ __device__ __forceinline__ double normalize(double *v) {
     return mag * inv;
   }
   mag = sqrt(mag);
+  bool ok = true;
+  const double y = recip_rn(mag, ok);
+  double q[ND];
 #pragma unroll
-  for (int i = 0; i < ND; ++i) v[i] /= mag;
+  for (int i = 0; i < ND; ++i) q[i] = div_rn(v[i], mag, y, ok);
+  if (!ok) {
+    asm volatile("" : "+d"(mag));  // a branch: not computed beside the fast path
+#pragma unroll
+    for (int i = 0; i < ND; ++i) q[i] = v[i] / mag;
+  }
+#pragma unroll
+  for (int i = 0; i < ND; ++i) v[i] = q[i];
   return mag;
 }
 
@@ -552,7 +736,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // Block-wide parallel cyclic reduction (Hockney, J. ACM 12:95-113, 1965;
 // Hockney & Jesshope, "Parallel Computers 2", 1988, sec. 5.4) of every
 // filament's tridiagonal system of the block at once, for the fast
-// integrator's blocks of long filaments: the rows laid out as solve_tridiag
+// integrator's blocks of long filaments: the rows laid out as thomas_twisted
 // takes them (row i of a filament at slot first + i: lower coefficient in
 // a[slot - 1], diagonal b, upper c, right-hand side d).  Each row thread
 // eliminates the unknowns s rows away on both sides (s = 1, 2, 4, ... below
@@ -604,11 +788,6 @@ __device__ __forceinline__ void pcr_block(double *a, double *b, double *c, doubl
   if (row) d[t] = rhs * recip_nr(dg);
 }
 
-// Rows of the longest system (bonds of the longest filament) above which the
-// fast 256- and 512-site integrators solve by pcr_block instead of Thomas
-// lanes.
-constexpr int kPcrMinRows = 32;
-
 template <int MAXC, bool FAST>
 struct IntegrateBounds {
   // The exact variant spills below 96 registers; the fast one fits 80, which
@@ -652,6 +831,11 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // sc), free between the two solves' uses.
   double *sdt = midstep ? srp : sT;  // det_t     2C
   double *sdb = sdt + 2 * C;         // det_b     2C
+  // The exact step's, where P1's inputs were: det_t and det_b over the bond
+  // forces (n + 1 values per filament of at least 3 sites), the tension
+  // matrix's elimination (den, inv, up; C each) over the bond torques.  The
+  // projection matrix's goes over srp, its solution over sdz.
+  double *xdt = sbF, *xdb = sbF + C + C / 2, *xden = sfr;
   double *sdz = sfp + 3 * C;    // full step: prefetched rebuild origin (3C), tracker (C)
   int *sflag = (int *)(sdz + 4 * C);            // C/2 renormalisation flags
   FilConst *sfil = (FilConst *)(sflag + C / 2); // the block's filaments
@@ -787,25 +971,18 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   if (FAST && MAXC > 128)
     for (int q = 0; q < nfb; ++q) max_rows = max(max_rows, sfil[q].n - 1);
   const bool pcr = FAST && MAXC > 128 && max_rows > kPcrMinRows;
-  // Sequential solves: the exact step keeps the reference's Thomas order on
-  // one lane per filament; the fast step solves from both ends on lanes
-  // 2q, 2q+1.
+  // Sequential solves of the fast step: from both ends on lanes 2q, 2q+1.
   auto solve_rows = [&](int lane_t) {
-    if (FAST) {
-      if (lane_t < 2 * nfb) {
-        const FilConst &f = sfil[lane_t >> 1];
-        const int fb0 = f.site0 - s0;
-        thomas_twisted(sa + fb0, sb + fb0, sc + fb0, sT + fb0, f.n - 1, (lane_t & 1) == 0);
-      }
-    } else if (lane_t < nfb) {
-      const int fb0 = sfil[lane_t].site0 - s0;
-      solve_tridiag<FAST>(sa + fb0, sb + fb0, sc + fb0, sT + fb0, sfil[lane_t].n - 1);
+    if (lane_t < 2 * nfb) {
+      const FilConst &f = sfil[lane_t >> 1];
+      const int fb0 = f.site0 - s0;
+      thomas_twisted(sa + fb0, sb + fb0, sc + fb0, sT + fb0, f.n - 1, (lane_t & 1) == 0);
     }
   };
   // Midstep determinants on warps the random-force solve leaves idle: lanes
   // from g_dt (forward) and g_db (backward), when three warp-aligned groups
   // fit in the block.
-  const int g_dt = ((FAST ? 2 * nfb : nfb) + 31) & ~31;
+  const int g_dt = (2 * nfb + 31) & ~31;
   const int g_db = g_dt + ((nfb + 31) & ~31);
   const bool dets_early = g_db + nfb <= C;
   if (active && j == n - 1) {
@@ -943,8 +1120,11 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
       d.fr[1][g] = fr[1];
       d.fr[2][g] = fr[2];
     }
-  } else if (midstep) {
-    if (k.stoch) {
+  } else if (!FAST) {
+    // The exact step: everything that the orientations alone decide -- noise,
+    // both matrices' eliminations, the determinants -- then the projection.
+    const bool noisy = midstep && k.stoch;
+    if (noisy) {
       if (active) {  // ConstructUnprojectedRandomForces (:518-548)
         uint32_t w[4];
         sc_host_philox4x32_10((uint32_t)j, (uint32_t)mcount, (uint32_t)(mcount >> 32), 0u,
@@ -953,12 +1133,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
 #pragma unroll
         for (int i = 0; i < ND; ++i)
           xi[i] = centered_uniform(w[i]);
-        if (FAST) {
-          // (t t^T) xi = (t . xi) t
-          const double txi = dotn<ND>(tn, xi);
-#pragma unroll
-          for (int i = 0; i < ND; ++i) xt[i] = txi * tn[i];
-        } else if (ND == 2) {
+        if (ND == 2) {
           xt[0] = tn[0] * tn[0] * xi[0] + tn[0] * tn[1] * xi[1];
           xt[1] = tn[1] * tn[1] * xi[1] + tn[0] * tn[1] * xi[0];
         } else {
@@ -969,6 +1144,77 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
           xt[2] = tn[2] * tn[2] * xi[2] + tn[0] * tn[2] * xi[0] +
                   tn[1] * tn[2] * xi[1];
         }
+#pragma unroll
+        for (int i = 0; i < ND; ++i)
+          fr[i] = fc.sperp * xi[i] + (fc.spar - fc.sperp) * xt[i];
+        for (int i = 0; i < 3; ++i) V(sfn, t, i) = fr[i];
+      }
+      __syncthreads();
+    } else if (!midstep && active) {
+      cp_async_wait_all();
+      if (k.stoch)
+        for (int i = 0; i < ND; ++i) fr[i] = V(sfp, t, i);
+    }
+    if (has_bond) {
+      // Tension matrix (:778-838): it holds no forces.
+      double tn2[3] = {V(stn, t + 1, 0), V(stn, t + 1, 1), V(stn, t + 1, 2)};
+      const double d1 = dotn<ND>(tn, u), d2 = dotn<ND>(tn2, u);
+      sb[t] = fc.two_igperp + fc.dgam * (d1 * d1 + d2 * d2);
+      if (j > 0) {
+        double u1[3] = {V(su, t - 1, 0), V(su, t - 1, 1), V(su, t - 1, 2)};
+        sa[t - 1] = fc.m1_igperp * dotn<ND>(u, u1) - fc.dgam * (dotn<ND>(tn, u1) * d1);
+      }
+      if (noisy) {  // GeometricallyProjectRandomForces (:550-599)
+        double tmp[3];
+#pragma unroll
+        for (int i = 0; i < ND; ++i) tmp[i] = V(sfn, t + 1, i) - fr[i];
+        sT[t] = dotn<ND>(tmp, u);
+      }
+    }
+    __syncthreads();
+    if (t < 2 * nfb) {
+      const int q = t >> 1, fb0 = sfil[q].site0 - s0;
+      const bool trail = (t & 1) != 0;
+      double *e = trail ? xden : srp;  // den, inv, up
+      factor_and_minors(trail, trail || noisy, scos + fb0, sa + fb0, sb + fb0, e + fb0,
+                        e + C + fb0, e + 2 * C + fb0, (trail ? xdb : xdt) + fb0 + q, sfil[q].n);
+    }
+    __syncthreads();
+    if (noisy && t < nfb) {
+      const int fb0 = sfil[t].site0 - s0;
+      tridiag_rhs<true>(scos + fb0, srp + fb0, srp + C + fb0, srp + 2 * C + fb0, sT + fb0,
+                        sdz + fb0, sfil[t].n - 1);
+    }
+    if (active && j < n - 2) {
+      const int dbase = base + lf;
+      const double ginv = scos[t] * xdt[dbase + j] * xdb[dbase + j + 3] / xdt[dbase + n - 1];
+      skeff[t] = div_by(fc.kappa + fc.l * ginv, fc.l2, fc.l2inv);
+    }
+    __syncthreads();
+    if (noisy && active) {
+#pragma unroll
+      for (int i = 0; i < ND; ++i) {
+        if (j < n - 1) fr[i] = fr[i] + sdz[t] * u[i];
+        if (j > 0) fr[i] = fr[i] - sdz[t - 1] * V(su, t - 1, i);
+      }
+      d.fr[0][g] = fr[0];  // the projected noise, reused by the full step
+      d.fr[1][g] = fr[1];
+      d.fr[2][g] = fr[2];
+    }
+  } else if (midstep) {
+    if (k.stoch) {
+      if (active) {  // ConstructUnprojectedRandomForces (:518-548)
+        uint32_t w[4];
+        sc_host_philox4x32_10((uint32_t)j, (uint32_t)mcount, (uint32_t)(mcount >> 32), 0u,
+                              s_seed, (uint32_t)fc.f_local, w);
+        double xi[3] = {0, 0, 0}, xt[3] = {0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < ND; ++i)
+          xi[i] = centered_uniform(w[i]);
+        // (t t^T) xi = (t . xi) t
+        const double txi = dotn<ND>(tn, xi);
+#pragma unroll
+        for (int i = 0; i < ND; ++i) xt[i] = txi * tn[i];
 #pragma unroll
         for (int i = 0; i < ND; ++i)
           fr[i] = fc.sperp * xi[i] + (fc.spar - fc.sperp) * xt[i];
@@ -1032,18 +1278,11 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // ---- P3: bending and metric forces (:608-776) ---------------------------
   // (The determinants do not share memory with the projection's solution,
   // which every thread has just read.)
-  if (!(dets_early && midstep && k.stoch && !pcr)) {
+  if (FAST && !(dets_early && midstep && k.stoch && !pcr)) {
     if (t < nfb) det_forward(sdt, scos, sfil[t], s0, t);
     else if (t >= C / 2 && t - C / 2 < nfb) det_backward(sdb, scos, sfil[t - C / 2], s0, t - C / 2);
     __syncthreads();
   }
-  if (!FAST && active && j < n - 2) {
-    const int dbase = base + lf;
-    const double det_g = sdt[dbase + n - 1];
-    double ginv = scos[t] * sdt[dbase + j] * sdb[dbase + j + 3] / det_g;
-    skeff[t] = (fc.kappa + fc.l * ginv) / fc.l2;
-  }
-  if (!FAST) __syncthreads();
   if (active && FAST) {
     // Each site forms the k_eff of the (up to) three joints its stencil
     // uses from the determinants and cosines, instead of reading them from
@@ -1181,35 +1420,47 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
 #pragma unroll
     for (int i = 0; i < ND; ++i) fdiff[i] = V(sbF, t + 1, i) - V(sbF, t, i);
     sT[t] = dotn<ND>(u, fdiff);
-    double tn2[3] = {V(stn, t + 1, 0), V(stn, t + 1, 1), V(stn, t + 1, 2)};
-    double d1 = dotn<ND>(tn, u);
-    double d2 = dotn<ND>(tn2, u);
-    sb[t] = fc.two_igperp + fc.dgam * (d1 * d1 + d2 * d2);
-    if (j > 0) {
-      double u1[3] = {V(su, t - 1, 0), V(su, t - 1, 1), V(su, t - 1, 2)};
-      double hu = fc.m1_igperp * dotn<ND>(u, u1) -
-                  fc.dgam * (dotn<ND>(tn, u1) * dotn<ND>(tn, u));
-      sc[t - 1] = hu;
-      sa[t - 1] = hu;
+    if (FAST) {
+      double tn2[3] = {V(stn, t + 1, 0), V(stn, t + 1, 1), V(stn, t + 1, 2)};
+      double d1 = dotn<ND>(tn, u);
+      double d2 = dotn<ND>(tn2, u);
+      sb[t] = fc.two_igperp + fc.dgam * (d1 * d1 + d2 * d2);
+      if (j > 0) {
+        double u1[3] = {V(su, t - 1, 0), V(su, t - 1, 1), V(su, t - 1, 2)};
+        double hu = fc.m1_igperp * dotn<ND>(u, u1) -
+                    fc.dgam * (dotn<ND>(tn, u1) * dotn<ND>(tn, u));
+        sc[t - 1] = hu;
+        sa[t - 1] = hu;
+      }
     }
   }
   __syncthreads();
-  if (pcr) pcr_block(sa, sb, sc, sT, has_bond, t, base, base + n - 2, max_rows);
-  else solve_rows(t);
+  if (!FAST) {
+    if (t < nfb) {
+      const int fb0 = sfil[t].site0 - s0;
+      tridiag_rhs<false>(sa + fb0, xden + fb0, xden + C + fb0, xden + 2 * C + fb0, sT + fb0,
+                         sc + fb0, sfil[t].n - 1);
+    }
+  } else if (pcr) {
+    pcr_block(sa, sb, sc, sT, has_bond, t, base, base + n - 2, max_rows);
+  } else {
+    solve_rows(t);
+  }
   __syncthreads();
+  const double *sx = FAST ? sT : sc;  // tensions
 
   // ---- P5: UpdateSitePositions (:840-927), CheckBondLengths (:934-951) ----
   if (active) {
     double fs[3];
     if (j == 0) {
 #pragma unroll
-      for (int i = 0; i < ND; ++i) fs[i] = sT[t] * u[i];
+      for (int i = 0; i < ND; ++i) fs[i] = sx[t] * u[i];
     } else if (j == n - 1) {
 #pragma unroll
-      for (int i = 0; i < ND; ++i) fs[i] = -sT[t - 1] * V(su, t - 1, i);
+      for (int i = 0; i < ND; ++i) fs[i] = -sx[t - 1] * V(su, t - 1, i);
     } else {
 #pragma unroll
-      for (int i = 0; i < ND; ++i) fs[i] = sT[t] * u[i] - sT[t - 1] * V(su, t - 1, i);
+      for (int i = 0; i < ND; ++i) fs[i] = sx[t] * u[i] - sx[t - 1] * V(su, t - 1, i);
     }
 #pragma unroll
     for (int i = 0; i < ND; ++i) F[i] += fs[i];
@@ -1254,7 +1505,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
       stretched = a < lo * lo || a > hi * hi;
     } else {
       a = sqrt(a);
-      double err = dabs(fc.l - a) / fc.l;
+      const double err = div_by(dabs(fc.l - a), fc.l, fc.linv);
       stretched = err > 1e-3;
     }
     if (stretched) sflag[lf] = 1;
@@ -1359,7 +1610,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     if (bad) atomicOr(d.status, ST_NAN);
     if (capture) {
       for (int i = 0; i < 3; ++i) d.cap_F[i][g] = F[i];
-      if (has_bond) d.cap_T[b] = sT[t];
+      if (has_bond) d.cap_T[b] = sx[t];
     }
     // Displacement tracking for the next query (Mesh::UpdateDrTot runs on
     // the filaments whose last update was a full step; each query adds the

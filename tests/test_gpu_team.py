@@ -1,0 +1,96 @@
+"""The team integrator (a warp's lanes per filament, one or two sites a lane)
+against the CPU oracle, bit for bit, at the sizes where its layout changes:
+filaments that fill a warp or leave one lane, the shortest ones, warps whose
+last filaments are missing, two sites a lane with odd and even site counts."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _lattice(n_dim, n_seg, side, seed, min_bond_length=0.666):
+    """Straight filaments on a grid with random directions: (system,
+    filaments, sites) for bond counts n_seg."""
+    rng = np.random.default_rng(seed)
+    n = len(n_seg)
+    per = int(np.ceil(n ** (1.0 / n_dim)))
+    cells = np.stack(np.meshgrid(*[np.arange(per)] * n_dim, indexing="ij"), -1).reshape(-1, n_dim)
+    length = np.maximum(n_seg * 1.5 * min_bond_length, 5.0)
+    sites = []
+    for i in range(n):
+        u = rng.normal(size=n_dim)
+        u /= np.linalg.norm(u)
+        head = np.zeros(3)
+        head[:n_dim] = (cells[i] + 0.5) * side / per - 0.5 * side
+        step = np.zeros(3)
+        step[:n_dim] = u * length[i] / n_seg[i]
+        sites.append(head + np.arange(n_seg[i] + 1)[:, None] * step)
+    system = dict(n_dim=n_dim, system_radius=0.5 * side, delta=1e-4, seed=seed)
+    fils = [dict(length=float(l) * (1 + 1e-12), persistence_length=100.0, diameter=1.0,
+                 min_bond_length=min_bond_length, friction_ratio=2.0) for l in length]
+    return system, fils, np.concatenate(sites)
+
+
+# (dimensions, bond counts, side): one site a lane ...
+CASES = {
+    "shortest": (3, [2] * 23, 40.0),
+    "full_warp": (3, [31, 31, 30, 5], 60.0),
+    "ragged": (2, [5, 31, 16, 7, 40, 9, 15, 16, 30, 6, 70, 5], 120.0),
+    # ... and two, where that saves more than half the warps of a full chip.
+    "two_odd_2d": (2, [16] * 3050, 900.0),
+    "two_even_3d": (3, [17] * 3001, 260.0),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_team_integrator_bitwise(name):
+    import simcore_b200 as sc
+    from checkers import Oracle
+    n_dim, n_seg, side = CASES[name]
+    system, fils, sites = _lattice(n_dim, np.array(n_seg), side, seed=5,
+                                   min_bond_length=2.0 if name == "shortest" else 0.666)
+    assert [sc.filament_n_bonds(f) for f in fils] == n_seg
+    ctx = sc.Context(system, fils, sites, precision="fp64")
+    oracle = Oracle(system, fils, sites)
+    for captured in (False, True):
+        (ctx.step_graph if captured else ctx.step)(4)
+        oracle.step(4)
+        assert np.array_equal(ctx.sites(), oracle.sites())
+        assert np.array_equal(ctx.random_forces(), oracle.random_forces())
+    ctx.close()
+    oracle.close()
+
+
+@pytest.mark.parametrize("name", ["full_warp", "two_odd_2d", "two_even_3d"])
+def test_fast_team_close_to_exact(name):
+    """Without noise the fast variant differs from the exact one by FP64
+    rounding alone: 1e-12 in the positions (about 100, rounding 1e-14, a few
+    steps of the implicit tension solve)."""
+    import simcore_b200 as sc
+    n_dim, n_seg, side = CASES[name]
+    system, fils, sites = _lattice(n_dim, np.array(n_seg), side, seed=6)
+    system = dict(system, stoch_flag=0)
+    got = []
+    for fast in (False, True):
+        ctx = sc.Context(system, fils, sites, precision="mixed")
+        ctx.set_fast_integrator(fast)
+        ctx.step(4)
+        got.append(ctx.sites())
+        ctx.close()
+    assert np.abs(got[0] - got[1]).max() <= 1e-12 * max(1.0, side / 100.0)
+
+
+def test_division_by_shared_reciprocal_special_values():
+    """Straight, unloaded filaments without noise: every right-hand side is
+    zero and the cosines are one, so the exact solves meet zero numerators."""
+    import simcore_b200 as sc
+    from checkers import Oracle
+    system, fils, sites = _lattice(3, np.array([7, 12, 31]), 60.0, seed=9)
+    system = dict(system, stoch_flag=0)
+    ctx = sc.Context(system, fils, sites, precision="fp64")
+    oracle = Oracle(system, fils, sites)
+    ctx.step(6)
+    oracle.step(6)
+    assert np.array_equal(ctx.sites(), oracle.sites())
+    ctx.close()
+    oracle.close()
