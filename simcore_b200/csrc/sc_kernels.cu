@@ -1347,6 +1347,7 @@ __global__ void k_loop_head(DevState d, cudaGraphConditionalHandle h,
 // with it.
 __global__ void k_loop_tail(DevState d, int stoch, cudaGraphConditionalHandle h,
                             cudaGraphConditionalHandle h_if, int decide) {
+  grid_dep_sync();
   const unsigned status = *d.status;  // the same word for every thread
   if (status & ST_LIST_OVERFLOW) {
     if (threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
@@ -1375,7 +1376,7 @@ int launch_loop_head(const DevState &d, cudaGraphConditionalHandle h,
 
 int launch_loop_tail(const DevState &d, int stoch, cudaGraphConditionalHandle h,
                      cudaGraphConditionalHandle h_if, int decide, cudaStream_t st) {
-  k_loop_tail<<<1, 256, 0, st>>>(d, stoch, h, h_if, decide);
+  launch_pdl(k_loop_tail, dim3(1), dim3(256), 0, st, d, stoch, h, h_if, decide);
   return 1;
 }
 
