@@ -1017,6 +1017,18 @@ static sc_status add_systems(sc_ctx *c, int nrep, const double *radius, const ui
                (size_t)std::max(sc::scan_temp_ints(rb.n_groups), sc::scan_temp_ints(2 * nbi))));
     CKS(dzero(&rb.cand_n, 1));
     CKS(dalloc(c, &rb.cand_start, nbi));
+    rb.grp_rep = nullptr;
+    if (nrep > 1) {
+      std::vector<int> grp_rep(rb.n_groups);
+      for (int r = 0; r < nrep; ++r) {
+        const sc::ReplicaConst &R = c->reps[r];
+        const int end = r + 1 < nrep ? c->reps[r + 1].cell0 / 32 : rb.n_groups;
+        for (int g = R.cell0 / 32; g < end; ++g) grp_rep[g] = r;
+      }
+      CKS(up(&tmp_i, grp_rep));
+      rb.grp_rep = tmp_i;
+      CK(cudaStreamSynchronize(c->st));  // grp_rep is pageable memory of this block
+    }
   }
   CKS(dzero(&d.e_off, nbi));
   CKS(dzero(&d.e_cnt, nbi));

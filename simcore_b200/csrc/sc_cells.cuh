@@ -10,18 +10,12 @@
 namespace sc {
 
 // CellList::FindCellCoords (src/cell_list.cpp:139-157) on the bond's scaled
-// position, recomputed exactly from its sites; the cell index within the
-// bond's system.
+// position, recomputed exactly from its sites r1, r2; the cell index within
+// the bond's system.
 template <int ND>
-__device__ __forceinline__ int bond_cell(const DevState &d, const ReplicaConst &R, int b,
-                                         int *xyz) {
-  int f = d.bond_fil[b];
-  int site = b + f;
-  double r1[3], r2[3], s[3], u[3], len;
-  for (int i = 0; i < 3; ++i) {
-    r1[i] = d.r[i][site];
-    r2[i] = d.r[i][site + 1];
-  }
+__device__ __forceinline__ int bond_cell_of(const DevState &d, const ReplicaConst &R,
+                                            const double *r1, const double *r2, int *xyz) {
+  double s[3], u[3], len;
   bond_from_sites<ND>(R.hinv, r1, r2, s, u, len);
   int c[3] = {0, 0, 0};
   bool bad = false;
@@ -42,6 +36,17 @@ __device__ __forceinline__ int bond_cell(const DevState &d, const ReplicaConst &
   xyz[1] = c[1];
   xyz[2] = c[2];
   return (c[0] * R.n1d + c[1]) * R.third + c[2];
+}
+template <int ND>
+__device__ __forceinline__ int bond_cell(const DevState &d, const ReplicaConst &R, int b,
+                                         int *xyz) {
+  const int site = b + d.bond_fil[b];
+  double r1[3], r2[3];
+  for (int i = 0; i < 3; ++i) {
+    r1[i] = d.r[i][site];
+    r2[i] = d.r[i][site + 1];
+  }
+  return bond_cell_of<ND>(d, R, r1, r2, xyz);
 }
 
 // Pairs that ProcessPairInteraction marks no_interaction and the first

@@ -63,7 +63,7 @@ int launch_csr(const DevState &d, int *deg, const int *deg_off, cudaStream_t st)
 // Scratch of a context's rebuild (sc_rebuild.cu).  Sizes: key, tmp, skey,
 // sval, pair_count, deg: nb; gcount: n_groups; gstart: n_groups + 1;
 // pair_off, deg_off: nb + 1; range: n_cells; occ: n_groups words;
-// scan_tmp: scan_temp_ints(max(n_groups, nb)).  gcount, deg, range and occ
+// scan_tmp: scan_temp_ints(max(n_groups, nb)); grp_rep: n_groups.  gcount, deg, range and occ
 // start zeroed.
 struct RebuildBufs {
   int n_groups;        // groups of 32 cells: n_cells / 32 (each system's cells
@@ -76,6 +76,7 @@ struct RebuildBufs {
   int *sval;           // sorted bond ids
   int2 *range;         // per cell: [start, end) in the sorted order
   unsigned *occ;       // per cell: occupied in the last rebuild of its system
+  const int *grp_rep;  // system of every group (several systems; else null)
   // Per sorted entry: the pairs of the cell it heads (0 elsewhere), then per
   // bond its pair entries; one array of 2 nb, scanned as one into 2 nb + 1
   // offsets (pair_count = counts, deg = counts + nb; pair_off = offsets,

