@@ -792,9 +792,12 @@ template <int MAXC, bool FAST>
 struct IntegrateBounds {
   // The exact variant spills below 96 registers; the fast one fits 80, which
   // also holds 4 blocks of 192 sites per SM (2 waves of 17-filament blocks
-  // for 20,000 11-site filaments on 148 SMs).
+  // for 20,000 11-site filaments on 148 SMs) and 3 of 256: latency-bound, it
+  // gains from the third (20,000 filaments of 5 to 200 bonds, those above 32
+  // sites: 303 us a launch with two blocks at 119 registers, 233 with three,
+  // for 24 bytes of spills).
   static constexpr int min_blocks =
-      MAXC <= 128 ? (FAST ? 6 : 5) : MAXC <= 192 ? (FAST ? 4 : 3) : MAXC <= 256 ? 2 : 1;
+      MAXC <= 128 ? (FAST ? 6 : 5) : MAXC <= 192 ? (FAST ? 4 : 3) : MAXC <= 256 ? (FAST ? 3 : 2) : 1;
 };
 
 // FUSE (fast mixed step only): each bond evaluates its own pairs
