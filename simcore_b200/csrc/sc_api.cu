@@ -365,10 +365,45 @@ sc_status maybe_rebuild(sc_ctx *c) {
   return rebuild(c);
 }
 
-// Integrator work units over the filaments in order: runs of whole filaments
-// of at most warp_sites sites each go to the team kernel (one warp, K sites a
-// lane), longer ones to the block kernel (runs of whole filaments up to C
-// sites per block).
+// Whole filaments `ids` into bins of `cap` by their sizes, best fit in order
+// of decreasing size (equal sizes in filament order): the bins' filaments.
+template <class Size>
+static std::vector<std::vector<int>> best_fit(std::vector<int> ids, int cap, Size &&size) {
+  std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return size(a) > size(b); });
+  std::vector<std::vector<int>> bins;
+  std::vector<std::vector<int>> room(cap + 1);  // bins by what they still hold
+  for (int f : ids) {
+    const int need = size(f);
+    int left = need;
+    while (left <= cap && room[left].empty()) ++left;
+    int bin;
+    if (left <= cap) {
+      bin = room[left].back();
+      room[left].pop_back();
+    } else {
+      left = cap;
+      bin = (int)bins.size();
+      bins.emplace_back();
+    }
+    bins[bin].push_back(f);
+    room[left - need].push_back(bin);
+  }
+  return bins;
+}
+
+// Integrator work units: filaments of at most warp_sites sites each go to the
+// team kernel (one warp, K sites a lane), longer ones to the block kernel (up
+// to C sites per block).  A unit never mixes systems (its displacement maximum
+// is one system's).  Equal filaments of one system fill the units in order;
+// others are packed by size, since runs of consecutive ones leave a third of a
+// 256-site block empty (20,000 filaments of 5 to 200 bonds: 233 us a launch for
+// those above 32 sites in runs, 173 packed; FP64 57.5 and 37.8 for 4,000 of 5 to
+// 100).  A filament's
+// results do not depend on its unit, but the fast integrator's blocks of more
+// than 128 sites draw and project the noise in FP64 when one of their
+// filaments has more than kPcrMinRows bonds: packed, all of them do (blk_wide)
+// if any filament has, and with short filaments in the blocks (warp_sites
+// below 32) the runs stay as they are.
 sc_status layout_integrator(sc_ctx *c) {
   const std::vector<int> &off = c->site_off;
   const int n = c->nf;
@@ -384,15 +419,21 @@ sc_status layout_integrator(sc_ctx *c) {
                 c->C);
   const int team_max = c->warp_sites;
   auto sites = [&](int f) { return off[f + 1] - off[f]; };
-  // A work unit never mixes systems (its displacement maximum is one
-  // system's).
-  auto same = [&](int f, int f0) { return c->fil_rep.empty() || c->fil_rep[f] == c->fil_rep[f0]; };
-  auto team_end = [&](int f0, int k) {  // past the filaments of the team warp that starts at f0
-    int f = f0, used = 0;
-    while (f < n && sites(f) <= team_max && same(f, f0) && used + (sites(f) + k - 1) / k <= 32)
-      used += (sites(f++) + k - 1) / k;
-    return f;
-  };
+  auto rep = [&](int f) { return c->fil_rep.empty() ? 0 : c->fil_rep[f]; };
+  bool equal = n > 0, one_system = true;
+  for (int f = 1; f < n; ++f) {
+    equal = equal && sites(f) == sites(0);
+    one_system = one_system && rep(f) == rep(0);
+  }
+  // Every system's filaments of each kind.
+  std::vector<std::vector<int>> shorts, longs;
+  for (int f = 0; f < n; ++f) {
+    if (f == 0 || rep(f) != rep(f - 1)) {
+      shorts.emplace_back();
+      longs.emplace_back();
+    }
+    (sites(f) <= team_max ? shorts : longs).back().push_back(f);
+  }
   // Sites per lane.  One is the shorter chain (100 x 21 sites, FP64: 12.8 us a
   // step against 19.1 with two), two fill the warps better (15,839 x 17
   // sites, FP64: 47.7 us against 73.7, with 5,280 warps instead of 15,839);
@@ -400,34 +441,53 @@ sc_status layout_integrator(sc_ctx *c) {
   // an SM instead of 20, so two pay where they save more than half the warps
   // (the margin covers 20,000 filaments of 5 to 32 sites, 1.9 times fewer:
   // 35 us with one, 50 with two) and one lane a site fills the chip at all.
-  long long warps[3] = {0, 0, 0};
+  std::vector<std::vector<int>> teams[3];
   for (int k = 1; k <= 2; ++k)
-    for (int f = 0; f < n;) {
-      if (sites(f) <= team_max) {
-        f = team_end(f, k);
-        ++warps[k];
-      } else {
-        ++f;
-      }
-    }
-  const int K = warps[1] > 148 * 20 && 4 * warps[1] >= 9 * warps[2] ? 2 : 1;
-  std::vector<int> blk_site0, blk_f0, blk_nf, blk_ns;
+    for (const auto &ids : shorts)
+      for (auto &bin : best_fit(ids, 32, [&](int f) { return (sites(f) + k - 1) / k; }))
+        teams[k].push_back(std::move(bin));
+  const int K = teams[1].size() > 148 * 20 && 4 * teams[1].size() >= 9 * teams[2].size() ? 2 : 1;
+  const bool uni = equal && one_system && sites(0) <= team_max;
   std::vector<int4> lanes;
-  bool uni = n > 0 && sites(0) <= team_max;
-  for (int f = 1; uni && f < n; ++f) uni = sites(f) == sites(0) && same(f, 0);
-  int f = 0;
-  while (f < n && !uni) {
-    const int s0 = off[f], f0 = f;
-    if (sites(f) <= team_max) {
-      f = team_end(f0, K);
+  if (!uni)
+    for (const auto &bin : teams[K]) {
       const size_t base = lanes.size();
-      for (int q = f0; q < f; ++q)
-        for (int j = 0; j < sites(q); j += K)
-          lanes.push_back(make_int4(off[q] + j, q, j | sites(q) << 16, (q - f0) | (f - f0) << 8));
+      for (size_t q = 0; q < bin.size(); ++q)
+        for (int j = 0; j < sites(bin[q]); j += K)
+          lanes.push_back(make_int4(off[bin[q]] + j, bin[q], j | sites(bin[q]) << 16,
+                                    (int)q | (int)bin.size() << 8));
       // Idle lanes name the warp's first site, of a filament without sites.
-      while (lanes.size() < base + 32) lanes.push_back(make_int4(s0, f0, 0, (f - f0) << 8));
-    } else {
-      while (f < n && sites(f) > team_max && same(f, f0) && off[f + 1] - s0 <= c->C) ++f;
+      while (lanes.size() < base + 32)
+        lanes.push_back(make_int4(off[bin[0]], bin[0], 0, (int)bin.size() << 8));
+    }
+  // Blocks: of packed ones, their filaments with their first slots, and every
+  // slot's site; of runs, their first site and filament.
+  const bool packed = !equal && (c->prec == 0 || c->warp_sites >= 32);
+  std::vector<int> blk_site0, blk_f0, blk_nf, blk_ns;
+  std::vector<int2> list;
+  std::vector<int4> slots;
+  for (const auto &ids : longs) {
+    if (packed) {
+      for (const auto &bin : best_fit(ids, c->C, sites)) {
+        blk_site0.push_back(0);
+        blk_f0.push_back((int)list.size());
+        blk_nf.push_back((int)bin.size());
+        int slot = 0;
+        for (size_t q = 0; q < bin.size(); ++q) {
+          list.push_back(make_int2(bin[q], slot));
+          for (int j = 0; j < sites(bin[q]); ++j)
+            slots.push_back(make_int4(off[bin[q]] + j, bin[q], j | sites(bin[q]) << 16, (int)q));
+          slot += sites(bin[q]);
+        }
+        blk_ns.push_back(slot);
+        slots.resize(blk_f0.size() * (size_t)c->C, make_int4(off[bin[0]], bin[0], 0, 0));
+      }
+      continue;
+    }
+    for (size_t i = 0; i < ids.size();) {
+      const int f0 = ids[i], s0 = off[f0];
+      int f = f0;
+      while (i < ids.size() && ids[i] == f && off[f + 1] - s0 <= c->C) ++i, ++f;
       blk_site0.push_back(s0);
       blk_f0.push_back(f0);
       blk_nf.push_back(f - f0);
@@ -436,33 +496,41 @@ sc_status layout_integrator(sc_ctx *c) {
   }
   DevState &d = c->d;
   for (const void *q : {(const void *)d.blk_site0, (const void *)d.blk_f0, (const void *)d.blk_nf,
-                        (const void *)d.blk_ns, (const void *)d.tm_lane})
+                        (const void *)d.blk_ns, (const void *)d.blk_list, (const void *)d.blk_slot,
+                        (const void *)d.tm_lane})
     dfree(c, const_cast<void *>(q));
   auto up = [&](auto **dst, const auto &v) -> sc_status {
     using T = typename std::remove_reference<decltype(v)>::type::value_type;
     T *q = nullptr;
+    *dst = nullptr;
     CKS(dalloc(c, &q, v.size()));
     if (!v.empty())
       CK(cudaMemcpyAsync(q, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c->st));
     *dst = q;
     return SC_OK;
   };
+  d.blk_list = nullptr;
+  d.blk_slot = nullptr;
   CKS(up(&d.blk_site0, blk_site0));
   CKS(up(&d.blk_f0, blk_f0));
   CKS(up(&d.blk_nf, blk_nf));
   CKS(up(&d.blk_ns, blk_ns));
   CKS(up(&d.tm_lane, lanes));
+  if (!slots.empty()) {
+    CKS(up(&d.blk_list, list));
+    CKS(up(&d.blk_slot, slots));
+  }
   CK(cudaStreamSynchronize(c->st));
+  d.blk_wide = packed && max_long - 1 > sc::kPcrMinRows ? 1 : 0;
   c->nblocks = (int)blk_f0.size();
   d.blk_maxf = 0;
   for (int v : blk_nf) d.blk_maxf = std::max(d.blk_maxf, v);
   // Equal filaments in equal blocks covering every filament: the kernel
   // indexes them by arithmetic.
   d.blk_uni_n = d.blk_uni_fpb = 0;
-  if (!blk_f0.empty() && n > 0) {
+  if (!blk_f0.empty() && equal) {
     const int nn = off[1] - off[0], fpb = blk_nf[0];
     bool buni = nn > 0 && fpb > 0 && (long long)blk_f0.size() == ((long long)n + fpb - 1) / fpb;
-    for (int q = 0; buni && q <= n; ++q) buni = off[q] == (long long)q * nn;
     for (size_t i = 0; buni && i < blk_f0.size(); ++i) {
       const long long f0 = (long long)i * fpb;
       buni = blk_f0[i] == f0 && blk_nf[i] == std::min<long long>(fpb, n - f0) &&

@@ -145,6 +145,12 @@ struct DevState {
   const int *blk_nf;       // per block: filament count
   const int *blk_ns;       // per block: site count
   int blk_maxf;            // most filaments in one block (shared-memory size)
+  // Packed blocks (null: runs of consecutive filaments): per block, from
+  // blk_f0, its filaments with their first slots; per slot its site, its
+  // filament, its index | filament sites << 16, its filament in the block.
+  const int2 *blk_list;
+  const int4 *blk_slot;
+  int blk_wide;            // a packed block's filament has more than kPcrMinRows bonds
   // Equal filaments of blk_uni_n sites, blk_uni_fpb to a block, every block
   // but the last full, sites numbered filament by filament from 0: blocks
   // and sites then find their filaments by arithmetic (0: read the tables).

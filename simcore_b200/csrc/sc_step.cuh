@@ -874,20 +874,28 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // Every global load the step needs is issued here, before the first
   // barrier: the filament constants, the renormalisation state and the
   // block's system constants, below the site state.
-  int pre_sw = 0, pre_nn = 0;
+  int pre_sw = 0, pre_nn = 0, fid = f0 + t;  // (thread t < nfb) the block's filament t
   if (t < nfb) {
-    sfil[t] = d.fil[f0 + t];
+    int slot = 0;
+    if (d.blk_slot) {
+      const int2 e = d.blk_list[f0 + t];
+      fid = e.x;
+      slot = e.y;
+    }
+    sfil[t] = d.fil[fid];
+    if (d.blk_slot) sfil[t].site0 = s0 + slot;  // a filament's first slot is site0 - s0
     sflag[t] = 0;
-    pre_sw = d.f_switch[f0 + t];
-    pre_nn = d.f_nnorm[f0 + t];
+    pre_sw = d.f_switch[fid];
+    pre_nn = d.f_nnorm[fid];
   }
   if (t < 10) {
-    const ReplicaConst &Rb = d.rep[d.nrep == 1 ? 0 : d.fil[f0].rep];
+    const int first = d.blk_slot ? d.blk_list[f0].x : f0;
+    const ReplicaConst &Rb = d.rep[d.nrep == 1 ? 0 : d.fil[first].rep];
     if (t < 9) s_hinv[t] = Rb.hinv[t];
     else s_seed = Rb.seed;
   }
   const bool active = t < count;
-  const int g = s0 + t;
+  int g = s0 + t;
   // The site's place in its filament comes from site_jn, so every load of
   // P0 is issued here, alongside the staging of the filament constants,
   // rather than after the barrier.
@@ -896,6 +904,12 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     lf = t / un;
     jn = (t - lf * un) | un << 16;
     f = f0 + lf;
+  } else if (active && d.blk_slot) {
+    const int4 e = d.blk_slot[(size_t)blk * C + t];
+    g = e.x;
+    f = e.y;
+    jn = e.z;
+    lf = e.w;
   } else if (active) {
     f = d.site_fil[g];
     jn = d.site_jn[g];
@@ -973,7 +987,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   int max_rows = 0;
   if (FAST && MAXC > 128)
     for (int q = 0; q < nfb; ++q) max_rows = max(max_rows, sfil[q].n - 1);
-  const bool pcr = FAST && MAXC > 128 && max_rows > kPcrMinRows;
+  const bool pcr = FAST && MAXC > 128 && (d.blk_wide || max_rows > kPcrMinRows);
   // Sequential solves of the fast step: from both ends on lanes 2q, 2q+1.
   auto solve_rows = [&](int lane_t) {
     if (lane_t < 2 * nfb) {
@@ -1516,15 +1530,14 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // Positions change below only in a block with a filament to renormalise.
   __syncthreads_or(stretched);
   if (t < nfb) {
-    const int fg = f0 + t;
     int sw = pre_sw, nnorm = pre_nn;
     if (sflag[t]) {
       sw = !sw;
       nnorm = 0;
     }
     nnorm++;
-    d.f_switch[fg] = sw;
-    d.f_nnorm[fg] = nnorm;
+    d.f_switch[fid] = sw;
+    d.f_nnorm[fid] = nnorm;
   }
   // The renormalised filament is rebuilt from one end along the bond
   // orientations just computed: from its first site when the switch turns

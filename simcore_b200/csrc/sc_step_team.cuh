@@ -194,10 +194,10 @@ __global__ void __launch_bounds__(kTeamWarps * 32, K == 1 ? 5 : 4)
   constexpr int S = M::S;
 
   // ---- the lane's sites: [j0, j0 + K) of its filament -----------------------
-  int f, lf, j0, n, g0, f0, nfw;
+  int f, lf, j0, n, g0, nfw;
   if (d.tm_uni_n > 0) {  // equal filaments: no table load
     const int L = d.tm_uni_lanes, fpw = d.tm_uni_fpw, un = d.tm_uni_n;
-    f0 = w * fpw;
+    const int f0 = w * fpw;
     nfw = min(fpw, d.nf - f0);
     lf = t / L;
     j0 = (t - lf * L) * K;
@@ -213,7 +213,6 @@ __global__ void __launch_bounds__(kTeamWarps * 32, K == 1 ? 5 : 4)
     n = q.z >> 16;
     lf = q.w & 0xff;
     nfw = q.w >> 8;
-    f0 = __shfl_sync(FULL, f, 0);
   }
   const int b0 = g0 - f;         // bond of the lane's first site
   const int slot0 = t * K;       // its slot
@@ -232,8 +231,12 @@ __global__ void __launch_bounds__(kTeamWarps * 32, K == 1 ? 5 : 4)
   double r[K][3], u[K][3];
   int e0 = 0, ec[2] = {0, 0};  // the lane's pair slots: first, per bond
   // (The filament constants first: everything below reads them.)
-  for (int i = t; i < nfw * (int)(sizeof(FilConst) / 16); i += 32)
-    cp_async16(sm + M::fil + 2 * i, reinterpret_cast<const double2 *>(d.fil + f0) + i);
+  if (act[0]) {
+    constexpr int words = (int)(sizeof(FilConst) / 16);
+    for (int i = j0 / K; i < words; i += (n + K - 1) / K)  // by the filament's own lanes
+      cp_async16(sm + M::fil + 2 * (words * lf + i),
+                 reinterpret_cast<const double2 *>(d.fil + f) + i);
+  }
   cp_async_commit();
   if (lead) sbase[lf] = sb0;
 #pragma unroll

@@ -94,3 +94,31 @@ def test_division_by_shared_reciprocal_special_values():
     assert np.array_equal(ctx.sites(), oracle.sites())
     ctx.close()
     oracle.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_packed_units_keep_systems_apart(precision):
+    """Uneven filaments are packed into warps and blocks by size, within their
+    system: each of two systems in one context gives the bits it gives alone
+    (long filaments in both precisions' blocks, a system without any)."""
+    import simcore_b200 as sc
+    parts = [_lattice(2, np.array([5, 40, 31, 70, 9, 35, 33, 100, 8, 32]), 330.0, seed=3),
+             _lattice(2, np.array([12, 7, 30, 5]), 90.0, seed=4)]
+    fils = parts[0][1] + parts[1][1]
+    sites = np.concatenate([parts[0][2], parts[1][2]])
+    replicas = [dict(system_radius=p[0]["system_radius"], seed=p[0]["seed"],
+                     n_filaments=len(p[1])) for p in parts]
+    both = sc.Context(parts[0][0], fils, sites, precision=precision, replicas=replicas)
+    both.step(3)
+    both.step_graph(4)
+    alone = []
+    for system, f, x in parts:
+        ctx = sc.Context(system, f, x, precision=precision)
+        # One block size for all: the mixed blocks' noise follows it.
+        ctx.set_integrator_layout(32, 128)
+        ctx.step(3)
+        ctx.step_graph(4)
+        alone.append(ctx.sites())
+        ctx.close()
+    assert np.array_equal(both.sites(), np.concatenate(alone))
+    both.close()
