@@ -636,8 +636,8 @@ __device__ __forceinline__ void thomas_twisted(T *a, const T *b, T *c, T *d, int
 // src/filament.cpp:627-660): det_t forward and det_b backward, each on its
 // own lane; filament q's values start at slot (first site) + q.
 __device__ __forceinline__ void det_forward(double *sdt, const double *scos, const FilConst &f,
-                                            int s0, int q) {
-  const int fb0 = f.site0 - s0, nn = f.n;
+                                            int fb0, int q) {
+  const int nn = f.n;
   double *dt = sdt + fb0 + q;
   const double *cs = scos + fb0;
   // The two previous values are carried in registers and each cosine is
@@ -656,8 +656,8 @@ __device__ __forceinline__ void det_forward(double *sdt, const double *scos, con
   }
 }
 __device__ __forceinline__ void det_backward(double *sdb, const double *scos, const FilConst &f,
-                                             int s0, int q) {
-  const int fb0 = f.site0 - s0, nn = f.n;
+                                             int fb0, int q) {
+  const int nn = f.n;
   double *db = sdb + fb0 + q;
   const double *cs = scos + fb0;
   double d2 = 1, d1 = 2;
@@ -723,6 +723,10 @@ __device__ __forceinline__ void cp_async8(double *smem_dst, const double *gsrc) 
   unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc));
 }
+__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc));
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::);
 }
@@ -730,64 +734,143 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// MAXC: largest block (sites) the instantiation is launched with; blocks
-// per SM requested so that the register budget leaves room for several
-// blocks in flight.
 // Block-wide parallel cyclic reduction (Hockney, J. ACM 12:95-113, 1965;
 // Hockney & Jesshope, "Parallel Computers 2", 1988, sec. 5.4) of every
 // filament's tridiagonal system of the block at once, for the fast
 // integrator's blocks of long filaments: the rows laid out as thomas_twisted
 // takes them (row i of a filament at slot first + i: lower coefficient in
-// a[slot - 1], diagonal b, upper c, right-hand side d).  Each row thread
-// eliminates the unknowns s rows away on both sides (s = 1, 2, 4, ... below
-// max_rows), exchanging rows through the same arrays; a coupling that
-// reaches past its filament's rows is zero at every step, so it is skipped.
-// Every thread of the block calls it (max_rows is uniform); the solution
-// ends in d.  O(log n) steps instead of the O(n) sequential elimination,
-// with other rounding (the exact integrator keeps the reference's Thomas).
-__device__ __forceinline__ void pcr_block(double *a, double *b, double *c, double *d, bool row,
-                                          int t, int first, int last, int max_rows) {
-  double lo = 0.0, dg = 1.0, up = 0.0, rhs = 0.0;
+// a[slot - 1], diagonal b, upper c, right-hand side d).  Each row thread,
+// its row scaled to a unit diagonal, eliminates the unknowns s rows away on
+// both sides (s = 1, 2, 4, ... below max_rows); a coupling that reaches past
+// its filament's rows is zero at every step, so it is skipped.  Rows are
+// exchanged through x (3 C) and a, c, d in turn, one barrier a step.  Every
+// thread of the block calls it (max_rows is uniform); the solution ends in d.
+// O(log n) steps instead of the O(n) sequential elimination, with other
+// rounding (the exact integrator keeps the reference's Thomas).  Bound by the
+// steps' latency: a step of 256-site blocks took about 620 cycles with two
+// barriers and two reciprocals, 470 now.
+__device__ __forceinline__ void pcr_block(double *a, const double *b, double *c, double *d,
+                                          double *x, int C, bool row, int t, int first, int last,
+                                          int max_rows) {
+  double lo = 0.0, up = 0.0, rhs = 0.0;
   if (row) {
-    lo = t > first ? a[t - 1] : 0.0;
-    dg = b[t];
-    up = t < last ? c[t] : 0.0;
-    rhs = d[t];
+    const double r = recip_nr(b[t]);
+    lo = t > first ? a[t - 1] * r : 0.0;
+    up = t < last ? c[t] * r : 0.0;
+    rhs = d[t] * r;
   }
-  for (int s = 1; s < max_rows; s <<= 1) {
-    __syncthreads();  // every read of the previous values is done
+  bool mine = false;  // the next exchange goes through a, c, d
+  for (int s = 1; s < max_rows; s <<= 1, mine = !mine) {
+    double *xl = mine ? a : x, *xu = mine ? c : x + C, *xr = mine ? d : x + 2 * C;
     if (row) {
-      a[t] = lo;
-      b[t] = dg;
-      c[t] = up;
-      d[t] = rhs;
+      xl[t] = lo;
+      xu[t] = up;
+      xr[t] = rhs;
     }
     __syncthreads();
     if (row) {
       const bool has_m = t - s >= first, has_p = t + s <= last;
-      double al = 0.0, ga = 0.0, ndg = dg, nrhs = rhs, nlo = 0.0, nup = 0.0;
+      double lm = 0.0, um = 0.0, rm = 0.0, lp = 0.0, upp = 0.0, rp = 0.0;
       if (has_m) {
-        al = -lo * recip_nr(b[t - s]);
-        ndg = fma(al, c[t - s], ndg);
-        nrhs = fma(al, d[t - s], nrhs);
-        nlo = al * a[t - s];
+        lm = xl[t - s];
+        um = xu[t - s];
+        rm = xr[t - s];
       }
       if (has_p) {
-        ga = -up * recip_nr(b[t + s]);
-        ndg = fma(ga, a[t + s], ndg);
-        nrhs = fma(ga, d[t + s], nrhs);
-        nup = ga * c[t + s];
+        lp = xl[t + s];
+        upp = xu[t + s];
+        rp = xr[t + s];
       }
-      lo = nlo;
-      up = nup;
-      dg = ndg;
-      rhs = nrhs;
+      const double r = recip_nr(fma(-lo, um, fma(-up, lp, 1.0)));
+      rhs = fma(-lo, rm, fma(-up, rp, rhs)) * r;
+      lo = -(lo * lm) * r;
+      up = -(up * upp) * r;
     }
   }
-  __syncthreads();
-  if (row) d[t] = rhs * recip_nr(dg);
+  __syncthreads();  // the last exchange may have read d
+  if (row) d[t] = rhs;
 }
 
+// Product of two 2 x 2 matrices (row major): c = a b.
+__device__ __forceinline__ void mul22(const double a[4], const double b[4], double c[4]) {
+  const double c0 = a[0] * b[0] + a[1] * b[2], c1 = a[0] * b[1] + a[1] * b[3];
+  const double c2 = a[2] * b[0] + a[3] * b[2], c3 = a[2] * b[1] + a[3] * b[3];
+  c[0] = c0;
+  c[1] = c1;
+  c[2] = c2;
+  c[3] = c3;
+}
+
+// Metric determinants (CalculateBendingForces, src/filament.cpp:627-660) of a
+// fast block's long filaments, as scans of 2 x 2 matrices over the sites:
+// joint j takes (x, y) to (2 x - cos^2 y, x), det_t from the tail, det_b from
+// the head.  Each warp scans its part of a filament by shuffles; the filament's
+// other warps enter through their totals in st (8 doubles a warp).  Joint j's
+// thread leaves cos det_t[j] det_b[j + 3] in sg, the last site's 1 / det_t[n - 1]
+// in sd[lf].  Every thread of the block calls it; followed by a barrier.  The
+// sequential recurrences took 7,100 of a 256-site block's 37,000 cycles, this
+// 3,800.
+__device__ __forceinline__ void minors_block(bool active, double cosv, int j, int n, int t,
+                                             double *st, double *sg, double *sd, int lf) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = t & 31, w = t >> 5, base = t - j;
+  const bool joint = active && j < n - 2;
+  const double c2 = cosv * cosv;
+  double P[4] = {1, 0, 0, 1}, B[4];
+  if (joint) {
+    P[0] = 2;
+    P[1] = -c2;
+    P[2] = 1;
+    P[3] = 0;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) B[i] = P[i];
+  for (int s = 1; s < 32; s <<= 1) {
+    double q[4], z[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      q[i] = __shfl_up_sync(FULL, P[i], s);
+      z[i] = __shfl_down_sync(FULL, B[i], s);
+    }
+    if (active && j >= s && lane >= s) mul22(P, q, P);
+    if (active && j + s < n && lane + s < 32) mul22(B, z, B);
+  }
+  double e[4], z[4];  // the warp's part before the joint, from either side
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (lane == 31) st[8 * w + i] = P[i];
+    if (lane == 0) st[8 * w + 4 + i] = B[i];
+    e[i] = __shfl_up_sync(FULL, P[i], 1);
+    z[i] = __shfl_down_sync(FULL, B[i], 1);
+  }
+  __syncthreads();
+  if (!active) return;
+  double x = 2.0, y = 1.0, p = 2.0, q = 1.0;  // (det_t[1], det_t[0]), (det_b[n-1], det_b[n])
+  for (int v = base >> 5; v < w; ++v) {
+    const double *m = st + 8 * v;
+    const double nx = m[0] * x + m[1] * y;
+    y = m[2] * x + m[3] * y;
+    x = nx;
+  }
+  for (int v = (base + n - 1) >> 5; v > w; --v) {
+    const double *m = st + 8 * v + 4;
+    const double np = m[0] * p + m[1] * q;
+    q = m[2] * p + m[3] * q;
+    p = np;
+  }
+  double tx = x, ty = y, bq = q;
+  if (lane > 0 && j > 0) {
+    tx = e[0] * x + e[1] * y;
+    ty = e[2] * x + e[3] * y;
+  }
+  if (lane < 31 && j + 1 < n) bq = z[2] * p + z[3] * q;
+  if (joint) sg[t] = cosv * ty * bq;
+  if (j == n - 1) sd[lf] = recip_nr(tx);
+}
+
+// MAXC: largest block (sites) the instantiation is launched with; blocks
+// per SM requested so that the register budget leaves room for several
+// blocks in flight.
 template <int MAXC, bool FAST>
 struct IntegrateBounds {
   // The exact variant spills below 96 registers; the fast one fits 80, which
@@ -927,9 +1010,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   int fsw = 0;  // the filament's renormalisation direction before this step
   if (active) {
     fsw = d.f_switch[f];
-    r[0] = d.r[0][g];
-    r[1] = d.r[1][g];
-    r[2] = d.r[2][g];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) r[i] = d.r[i][g];
     if (!midstep) {
       // The full step needs the midstep's positions and projected noise
       // later; fetch them now, in the background.
@@ -947,9 +1029,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   if (has_bond) {
     // Site orientation = orientation of its bond as Bond::ReInit left it
     // (Mesh::UpdateSiteOrientations, src/mesh.cpp:168-173).
-    u[0] = d.ub[0][b];
-    u[1] = d.ub[1][b];
-    u[2] = d.ub[2][b];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) u[i] = d.ub[i][b];
     if (!FUSE && interaction) {
       e0 = d.e_off[b];
       e1 = e0 + d.e_cnt[b];
@@ -969,9 +1050,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
       bond_pair_sum<ND, PREC>(d, b, e0, e1, bF, bT);
   }
   if (active && midstep) {  // Mesh::UpdatePrevPositions (src/mesh.cpp:175-182)
-    d.rp[0][g] = r[0];
-    d.rp[1][g] = r[1];
-    d.rp[2][g] = r[2];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) d.rp[i][g] = r[i];
   }
   if (has_bond) {
     for (int i = 0; i < 3; ++i) {
@@ -988,11 +1068,13 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   if (FAST && MAXC > 128)
     for (int q = 0; q < nfb; ++q) max_rows = max(max_rows, sfil[q].n - 1);
   const bool pcr = FAST && MAXC > 128 && (d.blk_wide || max_rows > kPcrMinRows);
+  // First slot of the block's filament q.
+  auto slot_of = [&](int q) { return sfil[q].site0 - s0; };
   // Sequential solves of the fast step: from both ends on lanes 2q, 2q+1.
   auto solve_rows = [&](int lane_t) {
     if (lane_t < 2 * nfb) {
       const FilConst &f = sfil[lane_t >> 1];
-      const int fb0 = f.site0 - s0;
+      const int fb0 = slot_of(lane_t >> 1);
       thomas_twisted(sa + fb0, sb + fb0, sc + fb0, sT + fb0, f.n - 1, (lane_t & 1) == 0);
     }
   };
@@ -1118,12 +1200,12 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     __syncthreads();
     if (t < 2 * nfb) {
       const FilConst &f = sfil[t >> 1];
-      const int fb0 = f.site0 - s0;
+      const int fb0 = slot_of(t >> 1);
       thomas_twisted(fa + fb0, fb + fb0, fcm + fb0, fT + fb0, f.n - 1, (t & 1) == 0);
     }
     if (dets_early) {  // the determinants, on lanes of other warps meanwhile
-      if (t >= g_dt && t - g_dt < nfb) det_forward(sdt, scos, sfil[t - g_dt], s0, t - g_dt);
-      else if (t >= g_db && t - g_db < nfb) det_backward(sdb, scos, sfil[t - g_db], s0, t - g_db);
+      if (t >= g_dt && t - g_dt < nfb) det_forward(sdt, scos, sfil[t - g_dt], slot_of(t - g_dt), t - g_dt);
+      else if (t >= g_db && t - g_db < nfb) det_backward(sdb, scos, sfil[t - g_db], slot_of(t - g_db), t - g_db);
     }
     __syncthreads();
     if (active) {
@@ -1133,9 +1215,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
         const float up = j > 0 ? (float)V(su, t - 1, i) : 0.f;
         fr[i] = (double)fmaf(tt, uf[i], fmaf(-tp, up, frf[i]));
       }
-      d.fr[0][g] = fr[0];  // the projected noise, reused by the full step
-      d.fr[1][g] = fr[1];
-      d.fr[2][g] = fr[2];
+#pragma unroll
+      for (int i = 0; i < ND; ++i) d.fr[i][g] = fr[i];  // the projected noise, for the full step
     }
   } else if (!FAST) {
     // The exact step: everything that the orientations alone decide -- noise,
@@ -1190,7 +1271,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     }
     __syncthreads();
     if (t < 2 * nfb) {
-      const int q = t >> 1, fb0 = sfil[q].site0 - s0;
+      const int q = t >> 1, fb0 = slot_of(q);
       const bool trail = (t & 1) != 0;
       double *e = trail ? xden : srp;  // den, inv, up
       factor_and_minors(trail, trail || noisy, scos + fb0, sa + fb0, sb + fb0, e + fb0,
@@ -1198,7 +1279,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     }
     __syncthreads();
     if (noisy && t < nfb) {
-      const int fb0 = sfil[t].site0 - s0;
+      const int fb0 = slot_of(t);
       tridiag_rhs<true>(scos + fb0, srp + fb0, srp + C + fb0, srp + 2 * C + fb0, sT + fb0,
                         sdz + fb0, sfil[t].n - 1);
     }
@@ -1214,9 +1295,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
         if (j < n - 1) fr[i] = fr[i] + sdz[t] * u[i];
         if (j > 0) fr[i] = fr[i] - sdz[t - 1] * V(su, t - 1, i);
       }
-      d.fr[0][g] = fr[0];  // the projected noise, reused by the full step
-      d.fr[1][g] = fr[1];
-      d.fr[2][g] = fr[2];
+#pragma unroll
+      for (int i = 0; i < ND; ++i) d.fr[i][g] = fr[i];  // the projected noise, for the full step
     }
   } else if (midstep) {
     if (k.stoch) {
@@ -1252,12 +1332,12 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
       }
       __syncthreads();
       if (pcr) {
-        pcr_block(sa, sb, sc, sT, has_bond, t, base, base + n - 2, max_rows);
+        pcr_block(sa, sb, sc, sT, sfr, C, has_bond, t, base, base + n - 2, max_rows);
       } else {
         solve_rows(t);
         if (dets_early) {  // the determinants, on lanes of other warps meanwhile
-          if (t >= g_dt && t - g_dt < nfb) det_forward(sdt, scos, sfil[t - g_dt], s0, t - g_dt);
-          else if (t >= g_db && t - g_db < nfb) det_backward(sdb, scos, sfil[t - g_db], s0, t - g_db);
+          if (t >= g_dt && t - g_dt < nfb) det_forward(sdt, scos, sfil[t - g_dt], slot_of(t - g_dt), t - g_dt);
+          else if (t >= g_db && t - g_db < nfb) det_backward(sdb, scos, sfil[t - g_db], slot_of(t - g_db), t - g_db);
         }
       }
       __syncthreads();
@@ -1276,9 +1356,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
         }
 #pragma unroll
         for (int i = 0; i < ND; ++i) fr[i] = fp[i];
-        d.fr[0][g] = fr[0];  // the projected noise, reused by the full step
-        d.fr[1][g] = fr[1];
-        d.fr[2][g] = fr[2];
+#pragma unroll
+        for (int i = 0; i < ND; ++i) d.fr[i][g] = fr[i];  // the projected noise, for the full step
       }
     }
   } else if (active) {
@@ -1295,9 +1374,15 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // ---- P3: bending and metric forces (:608-776) ---------------------------
   // (The determinants do not share memory with the projection's solution,
   // which every thread has just read.)
-  if (FAST && !(dets_early && midstep && k.stoch && !pcr)) {
-    if (t < nfb) det_forward(sdt, scos, sfil[t], s0, t);
-    else if (t >= C / 2 && t - C / 2 < nfb) det_backward(sdb, scos, sfil[t - C / 2], s0, t - C / 2);
+  // (Blocks of long filaments: over srp in midsteps, sT and sa in full ones.)
+  double *sdet = midstep ? srp + C : sa;
+  if (FAST && pcr) {
+    minors_block(active, active && j < n - 2 ? scos[t] : 0.0, j, n, t, midstep ? srp : sT, skeff,
+                 sdet, lf);
+    __syncthreads();
+  } else if (FAST && !(dets_early && midstep && k.stoch)) {
+    if (t < nfb) det_forward(sdt, scos, sfil[t], slot_of(t), t);
+    else if (t >= C / 2 && t - C / 2 < nfb) det_backward(sdb, scos, sfil[t - C / 2], slot_of(t - C / 2), t - C / 2);
     __syncthreads();
   }
   if (active && FAST) {
@@ -1305,9 +1390,10 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     // uses from the determinants and cosines, instead of reading them from
     // a barrier later.
     const int dbase = base + lf;
-    const double rdet = recip_nr(sdt[dbase + n - 1]), rl2 = recip_nr(fc.l2);
+    const double rdet = pcr ? sdet[lf] : recip_nr(sdt[dbase + n - 1]), rl2 = recip_nr(fc.l2);
     auto keff_at = [&](int jj) {
-      const double ginv = scos[base + jj] * sdt[dbase + jj] * sdb[dbase + jj + 3] * rdet;
+      const double ginv =
+          (pcr ? skeff[base + jj] : scos[base + jj] * sdt[dbase + jj] * sdb[dbase + jj + 3]) * rdet;
       return (fc.kappa + fc.l * ginv) * rl2;
     };
     // (I - u2 u2^T) u1 = u1 - (u1 . u2) u2 with the cosines of
@@ -1454,12 +1540,12 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   __syncthreads();
   if (!FAST) {
     if (t < nfb) {
-      const int fb0 = sfil[t].site0 - s0;
+      const int fb0 = slot_of(t);
       tridiag_rhs<false>(sa + fb0, xden + fb0, xden + C + fb0, xden + 2 * C + fb0, sT + fb0,
                          sc + fb0, sfil[t].n - 1);
     }
   } else if (pcr) {
-    pcr_block(sa, sb, sc, sT, has_bond, t, base, base + n - 2, max_rows);
+    pcr_block(sa, sb, sc, sT, sfr, C, has_bond, t, base, base + n - 2, max_rows);
   } else {
     solve_rows(t);
   }
@@ -1613,13 +1699,11 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
         s[i] -= nint(s[i]);
       }
       store_geom<ND>(d, 1 - rbuf, b, s, ub, len, PREC);
-      d.ub[0][b] = ub[0];
-      d.ub[1][b] = ub[1];
-      d.ub[2][b] = ub[2];
+#pragma unroll
+      for (int i = 0; i < ND; ++i) d.ub[i][b] = ub[i];
     }
-    d.r[0][g] = r[0];
-    d.r[1][g] = r[1];
-    d.r[2][g] = r[2];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) d.r[i][g] = r[i];
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < ND; ++i) bad |= !isfinite(r[i]);

@@ -153,21 +153,6 @@ __device__ __forceinline__ void team_pair_sum(const DevState &d, int b0, const b
   }
 }
 
-// Product of two 2 x 2 matrices (row major): c = a b.
-__device__ __forceinline__ void mul22(const double a[4], const double b[4], double c[4]) {
-  const double c0 = a[0] * b[0] + a[1] * b[2], c1 = a[0] * b[1] + a[1] * b[3];
-  const double c2 = a[2] * b[0] + a[3] * b[2], c3 = a[2] * b[1] + a[3] * b[3];
-  c[0] = c0;
-  c[1] = c1;
-  c[2] = c2;
-  c[3] = c3;
-}
-
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc));
-}
-
 // FUSE (fast mixed step only): each bond evaluates its own pairs
 // (bond_pair_eval_sum) instead of summing the pair stage's slots.
 template <int ND, int PREC, bool FAST, int K, bool FUSE = false>
