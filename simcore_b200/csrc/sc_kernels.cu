@@ -840,9 +840,9 @@ template <int ND>
 __global__ void __launch_bounds__(128) k_tether(SysConst k, DevState d) {
   grid_dep_sync();
   const int A = blockIdx.x * blockDim.x + threadIdx.x, a = A & 1;  // the anchor; link A / 2
+  const unsigned lanes = __ballot_sync(0xffffffffu, A < 2 * d.nx);
   if (A >= 2 * d.nx) return;  // pairs of lanes together
   if (*d.status & ST_LIST_OVERFLOW) return;  // the step stopped at its rebuild
-  const unsigned pair = 3u << ((threadIdx.x & 31) & 30);
   const int f = d.xl_fil[A];
   const FilConst &fc = d.fil[f];
   const int nbf = fc.n - 1, b0 = fc.site0 - f;
@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(128) k_tether(SysConst k, DevState d) {
   double dr[3] = {0, 0, 0}, dr2 = 0.0, ft[3] = {0, 0, 0}, ds[3] = {0, 0, 0};
 #pragma unroll
   for (int i = 0; i < ND; ++i) {
-    const double other = __shfl_xor_sync(pair, sp[i], 1);
+    const double other = __shfl_xor_sync(lanes, sp[i], 1);
     ds[i] = a == 0 ? other - sp[i] : sp[i] - other;  // anchor 1 - anchor 0
     ds[i] -= nint(ds[i]);
   }
