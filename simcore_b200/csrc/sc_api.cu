@@ -69,13 +69,19 @@ sc_status check_status(sc_ctx *c) {
   return SC_OK;
 }
 
-// Reads the status word and every system's displacement maximum.
+sc::HostReport host_report(sc_ctx *c) {
+  return sc::HostReport{c->h_loop, c->hb->rebuilds, &c->hb->status, c->h_dr, c->h_np};
+}
+
+// Reads the status word, every system's displacement maximum and pair count.
 sc_status readback(sc_ctx *c) {
-  if (c->d.nrep > 0)
-    CK(cudaMemcpyAsync(c->h_dr, c->d.dr_max_bits, sizeof(unsigned long long) * c->d.nrep,
-                       cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(&c->hb->status, c->d.status, sizeof(unsigned),
-                     cudaMemcpyDeviceToHost, c->st));
+  if (c->d.nrep > 0) {
+    c->launches += sc::launch_report(c->d, host_report(c), 0, c->st);
+    CK(cudaGetLastError());
+  } else {  // nothing loaded yet
+    CK(cudaMemcpyAsync(&c->hb->status, c->d.status, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                       c->st));
+  }
   CK(cudaStreamSynchronize(c->st));
   return check_status(c);
 }
@@ -259,16 +265,24 @@ sc_status ensure_pair_capacity(sc_ctx *c, long long need) {
   return upload_reps(c);
 }
 
-// Pair counts of every system (device values); c->np is their total.
+// The pair counts that h_np received; c->np is their total.  They hold until
+// the next rebuild, which every caller follows with the counts' readback, and
+// a restore.
+void take_pair_count(sc_ctx *c) {
+  c->np = 0;
+  for (size_t r = 0; r < c->reps.size(); ++r) {
+    c->np_rep[r] = c->h_np[r];
+    c->np += std::min(c->h_np[r], c->reps[r].pcap);
+  }
+  c->np_known = true;
+}
+
+// Pair counts of every system (device values).
 sc_status sync_pair_count(sc_ctx *c) {
   const int nrep = c->d.nrep;
   CK(cudaMemcpyAsync(c->h_np, c->d.np_rep, sizeof(int) * nrep, cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  c->np = 0;
-  for (int r = 0; r < nrep; ++r) {
-    c->np_rep[r] = c->h_np[r];
-    c->np += std::min(c->h_np[r], c->reps[r].pcap);
-  }
+  take_pair_count(c);
   return SC_OK;
 }
 
@@ -280,6 +294,7 @@ sc_status sync_pair_count(sc_ctx *c) {
 void rebuild_enqueue(sc_ctx *c, bool first_in_graph) {
   const long long before = c->launches;
   const DevState &d = c->d;
+  c->np_known = false;
   if (c->desc.interaction_flag)
     c->launches += sc::launch_rebuild(c->k, d, c->rb, c->prec, c->st, first_in_graph);
   else

@@ -115,11 +115,12 @@ struct sc_ctx {
   unsigned long long *h_dr = nullptr;  // per system displacement maxima
   int *h_np = nullptr;                 // per system pair counts
   int *h_due = nullptr;                // per system rebuild flags
+  bool np_known = false;               // np and np_rep are the device's counts
 
   // CUDA graph: a WHILE loop of BD steps (sc_step_graph)
   cudaGraphExec_t graph_exec = nullptr;
   int graph_rbuf = -1;             // geometry buffer parity the graph was built for
-  int *h_loop = nullptr;           // pinned loop count
+  int *h_loop = nullptr;           // pinned: BD steps to do, left undone
 
   // optional per-launch timing of the step kernel (host-driven path)
   long long rebuild_kernels = 0;    // kernels in one rebuild sequence
@@ -198,6 +199,7 @@ void invert_sym_3d(const double *a, double *b);
 void filament_length(const sc_filament_params &p, double *length, int *n_bonds);
 // Status word -> sc_status; readback copies it (and the displacement maxima).
 sc_status check_status(sc_ctx *c);
+sc::HostReport host_report(sc_ctx *c);
 sc_status readback(sc_ctx *c);
 void drop_graph(sc_ctx *c);
 sc_status upload_reps(sc_ctx *c);
@@ -208,6 +210,7 @@ void install_store(sc_ctx *c, const PairStore &q);
 sc_status alloc_store(sc_ctx *c, long long total, PairStore &q);
 sc_status layout_pairs(sc_ctx *c, const std::vector<long long> &caps);
 sc_status ensure_pair_capacity(sc_ctx *c, long long need);
+void take_pair_count(sc_ctx *c);
 sc_status sync_pair_count(sc_ctx *c);
 // Pair-list rebuild (InteractionManager::UpdateInteractions).
 void rebuild_enqueue(sc_ctx *c, bool first_in_graph = false);

@@ -8,7 +8,7 @@ extern "C" {
 
 // Captures one graph: head (loop condition, first rebuild decision) ->
 // WHILE (loop_count > 0) { IF(rebuild) -> midstep -> full step -> tail (next
-// rebuild decision) }.  Built for the current geometry-buffer parity; every
+// rebuild decision) } -> report to the host.  Built for the current geometry-buffer parity; every
 // BD step returns the parity to where it started.
 static sc_status build_graph(sc_ctx *c) {
   drop_graph(c);
@@ -22,7 +22,7 @@ static sc_status build_graph(sc_ctx *c) {
   if (interaction) CK(cudaGraphConditionalHandleCreate(&h_if, g, 0, 0));
   // head kernel: sets the loop condition and decides the first rebuild
   CK(cudaStreamBeginCaptureToGraph(c->st, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-  sc::launch_loop_head(c->d, h_loop, h_if, interaction, c->st);
+  sc::launch_loop_head(c->d, host_report(c), h_loop, h_if, interaction, c->st);
   cudaStreamCaptureStatus cs;
   const cudaGraphNode_t *deps = nullptr;
   size_t ndeps = 0;
@@ -88,6 +88,10 @@ static sc_status build_graph(sc_ctx *c) {
   }
   sc::launch_loop_tail(c->d, c->desc.stoch_flag ? 1 : 0, h_loop, h_if, interaction, c->st);
   CK(cudaStreamEndCapture(c->st, &body));
+  // What the host reads afterwards.
+  CK(cudaStreamBeginCaptureToGraph(c->st, g, &wnode, nullptr, 1, cudaStreamCaptureModeRelaxed));
+  sc::launch_report(c->d, host_report(c), 1, c->st);
+  CK(cudaStreamEndCapture(c->st, &g));
   CK(cudaGetLastError());
   cudaError_t e = cudaGraphInstantiate(&c->graph_exec, g, 0);
   cudaGraphDestroy(g);
@@ -111,7 +115,7 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
   if (bd > 0) {
     CKS(thermo_reserve(c, 2 * (long long)bd));
     // The list must have room to grow by half before a captured run.
-    CKS(sync_pair_count(c));
+    if (!c->np_known) CKS(sync_pair_count(c));
     if (c->reps.size() == 1 && c->np + c->np / 2 > c->pcap)
       CKS(ensure_pair_capacity(c, c->np + c->np / 2));
     if (!c->gev0) {
@@ -125,24 +129,16 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
     for (int attempt = 0; bd > 0; ++attempt) {
       if (attempt == 8) return fail(c, SC_ERR_LIST_OVERFLOW, "pair list kept overflowing inside captured runs");
       if (!c->graph_exec || c->graph_rbuf != c->rbuf) CKS(build_graph(c));
+      // The head reads the step count and the last node writes everything
+      // the host looks at, both in pinned memory: no copies, one
+      // synchronisation per launch.
       *c->h_loop = bd;
-      CK(cudaMemcpyAsync(c->d.loop_count, c->h_loop, sizeof(int), cudaMemcpyHostToDevice, c->st));
-      // Every readback goes to pinned memory: one synchronisation per launch.
-      CK(cudaMemcpyAsync(&c->hb->rebuilds[0], c->d.n_rebuilds, sizeof(long long),
-                         cudaMemcpyDeviceToHost, c->st));
       CK(cudaEventRecord(c->gev0, c->st));
       CK(cudaGraphLaunch(c->graph_exec, c->st));
       CK(cudaEventRecord(c->gev1, c->st));
-      CK(cudaMemcpyAsync(&c->hb->rebuilds[1], c->d.n_rebuilds, sizeof(long long),
-                         cudaMemcpyDeviceToHost, c->st));
-      CK(cudaMemcpyAsync(c->h_loop, c->d.loop_count, sizeof(int), cudaMemcpyDeviceToHost, c->st));
       c->pairs_ready = false;
-      CK(cudaMemcpyAsync(&c->hb->status, c->d.status, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                         c->st));
-      if (c->d.nrep > 0)  // the displacement maxima too (readback's copies)
-        CK(cudaMemcpyAsync(c->h_dr, c->d.dr_max_bits, sizeof(unsigned long long) * c->d.nrep,
-                           cudaMemcpyDeviceToHost, c->st));
       CK(cudaStreamSynchronize(c->st));
+      take_pair_count(c);
       const unsigned st = c->hb->status;
       const long long nr0 = c->hb->rebuilds[0], nr1 = c->hb->rebuilds[1];
       const bool overflow = (st & sc::ST_LIST_OVERFLOW) != 0u;
@@ -156,7 +152,7 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
         CK(cudaEventElapsedTime(&ms, c->gev0, c->gev1));
         c->graph_ms += ms;
       }
-      // Kernels the graph ran: loop head, per BD step the two tether
+      // Kernels the graph ran: loop head and report, per BD step the two tether
       // kernels (mesh lambdas, anchor forces) + 2 steps + tail (the stopped
       // step's too), per rebuild the captured sequence.  A step is its pair
       // kernel (unless fused; near-parallel pairs are evaluated in place),
@@ -167,7 +163,7 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
               ? 1 + (c->d.nx ? 2 : 0) +
                     2 * ((c->graph_fused ? 0 : 1) + int_l + (c->k.thermo ? 1 : 0))
               : 1 + 2 * int_l;
-      c->launches += 1 + (long long)(done + (overflow ? 1 : 0)) * per_bd +
+      c->launches += 2 + (long long)(done + (overflow ? 1 : 0)) * per_bd +
                      (nr1 - nr0) * c->rebuild_kernels;
       bd -= done;
       if (!overflow) {

@@ -1316,12 +1316,30 @@ __device__ void decide_systems(const DevState &d, cudaGraphConditionalHandle h_i
   if (threadIdx.x == 0) cudaGraphSetConditional(h_if, any ? 1u : 0u);
 }
 
-// Start of a graph loop: the loop condition and the first step's rebuild
-// decision.
-__global__ void k_loop_head(DevState d, cudaGraphConditionalHandle h,
+// Start of a graph loop: the steps to do, the loop condition and the first
+// step's rebuild decision.
+__global__ void k_loop_head(DevState d, HostReport out, cudaGraphConditionalHandle h,
                             cudaGraphConditionalHandle h_if, int decide) {
   if (decide) decide_systems(d, h_if);
-  if (threadIdx.x == 0) cudaGraphSetConditional(h, *d.loop_count > 0 ? 1u : 0u);
+  if (threadIdx.x == 0) {
+    const int left = *(volatile int *)out.loop;
+    *d.loop_count = left;
+    out.rebuilds[0] = *d.n_rebuilds;
+    cudaGraphSetConditional(h, left > 0 ? 1u : 0u);
+  }
+}
+
+__global__ void k_report(DevState d, HostReport out, int graph) {
+  for (int r = threadIdx.x; r < d.nrep; r += blockDim.x) {
+    out.dr[r] = d.dr_max_bits[r];
+    out.np[r] = d.np_rep[r];
+  }
+  if (threadIdx.x != 0) return;
+  *out.status = *d.status;
+  if (graph) {
+    *out.loop = *d.loop_count;
+    out.rebuilds[1] = *d.n_rebuilds;
+  }
 }
 
 // End of one BD step (midstep + full step) of a graph loop: advances the
@@ -1353,9 +1371,14 @@ __global__ void k_advance_mcount(DevState d) {
   *d.mcount += 1ull;
 }
 
-int launch_loop_head(const DevState &d, cudaGraphConditionalHandle h,
+int launch_loop_head(const DevState &d, const HostReport &out, cudaGraphConditionalHandle h,
                      cudaGraphConditionalHandle h_if, int decide, cudaStream_t st) {
-  k_loop_head<<<1, 256, 0, st>>>(d, h, h_if, decide);
+  k_loop_head<<<1, 256, 0, st>>>(d, out, h, h_if, decide);
+  return 1;
+}
+
+int launch_report(const DevState &d, const HostReport &out, int graph, cudaStream_t st) {
+  k_report<<<1, 256, 0, st>>>(d, out, graph);
   return 1;
 }
 

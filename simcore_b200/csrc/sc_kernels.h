@@ -98,10 +98,22 @@ struct RebuildBufs {
 // body (launched without the programmatic-dependence attribute).
 int launch_rebuild(const SysConst &k, const DevState &d, const RebuildBufs &rb, int prec,
                    cudaStream_t st, bool first_in_graph);
+// What the host reads after a launch, in pinned memory that the device writes
+// itself (a handful of small copies and their gaps otherwise).
+struct HostReport {
+  int *loop;             // graph launches: BD steps to do (in), left undone (out)
+  long long *rebuilds;   // graph launches: rebuild passes before and after
+  unsigned *status;
+  unsigned long long *dr;  // per system: displacement maximum
+  int *np;                 // per system: pairs
+};
+// graph: also the loop's remaining steps and the rebuild passes, for a captured
+// run's end.
+int launch_report(const DevState &d, const HostReport &out, int graph, cudaStream_t st);
 // Graph loop control: the head sets the WHILE condition h and, with
 // `decide`, the first step's rebuild decision (IF condition h_if); the tail
 // ends a BD step and decides the next step's rebuild.
-int launch_loop_head(const DevState &d, cudaGraphConditionalHandle h,
+int launch_loop_head(const DevState &d, const HostReport &h_out, cudaGraphConditionalHandle h,
                      cudaGraphConditionalHandle h_if, int decide, cudaStream_t st);
 int launch_loop_tail(const DevState &d, int stoch, cudaGraphConditionalHandle h,
                      cudaGraphConditionalHandle h_if, int decide, cudaStream_t st);
