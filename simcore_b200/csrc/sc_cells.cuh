@@ -9,14 +9,11 @@
 
 namespace sc {
 
-// CellList::FindCellCoords (src/cell_list.cpp:139-157) on the bond's scaled
-// position, recomputed exactly from its sites r1, r2; the cell index within
-// the bond's system.
+// CellList::FindCellCoords (src/cell_list.cpp:139-157) on a bond's scaled
+// position; the cell index within the bond's system.
 template <int ND>
-__device__ __forceinline__ int bond_cell_of(const DevState &d, const ReplicaConst &R,
-                                            const double *r1, const double *r2, int *xyz) {
-  double s[3], u[3], len;
-  bond_from_sites<ND>(R.hinv, r1, r2, s, u, len);
+__device__ __forceinline__ int cell_of_scaled(const DevState &d, const ReplicaConst &R,
+                                              const double *s, int *xyz) {
   int c[3] = {0, 0, 0};
   bool bad = false;
 #pragma unroll
@@ -36,6 +33,15 @@ __device__ __forceinline__ int bond_cell_of(const DevState &d, const ReplicaCons
   xyz[1] = c[1];
   xyz[2] = c[2];
   return (c[0] * R.n1d + c[1]) * R.third + c[2];
+}
+// The same from the bond's sites r1, r2, its scaled position recomputed
+// exactly, or from the bond's index.
+template <int ND>
+__device__ __forceinline__ int bond_cell_of(const DevState &d, const ReplicaConst &R,
+                                            const double *r1, const double *r2, int *xyz) {
+  double s[3], u[3], len;
+  bond_from_sites<ND>(R.hinv, r1, r2, s, u, len);
+  return cell_of_scaled<ND>(d, R, s, xyz);
 }
 template <int ND>
 __device__ __forceinline__ int bond_cell(const DevState &d, const ReplicaConst &R, int b,

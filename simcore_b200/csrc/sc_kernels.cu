@@ -1,10 +1,10 @@
 // Device kernels of the B200 filament step.  Compiled with --fmad=false
 // (see sc_common.cuh).
 //
-//   cell list      k_bin_count, k_bin_scatter, k_cell_sort_count,
+//   cell list      k_bin_scatter, k_cell_sort_count,
 //                  k_pair_emit   (CellList + Cell, src/cell_list.cpp,
 //                                 src/cell.cpp)
-//   pair CSR       k_csr_offsets, k_csr_fill, k_csr_sort_pos (per-bond pair
+//   pair CSR       k_csr_fill, k_csr_sort_pos (per-bond pair
 //                  entries in list order, for the reference's serial
 //                  scatter order)
 //   pair forces    k_pair_eval   (InteractionManager::CalculatePairInteractions,
@@ -58,34 +58,6 @@ __global__ void k_bond_cells(SysConst k, DevState d, int *xyz) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= d.nb) return;
   bond_cell<ND>(d, d.rep[rep_of_bond(d, b)], b, xyz + 3 * (size_t)b);
-}
-
-// Bonds of the systems whose list is rebuilt in this pass: global cell key
-// and cell counts.
-template <int ND>
-__global__ void k_bin_count(SysConst k, DevState d, int *key, int *cell_count) {
-  grid_dep_sync();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = b < d.nb;
-  int c = -1;
-  if (active) {
-    const int r = rep_of_bond(d, b);
-    if (d.due[r]) {
-      const ReplicaConst &R = d.rep[r];
-      int xyz[3];
-      c = R.cell0 + bond_cell<ND>(d, R, b, xyz);
-      key[b] = c;
-    } else {
-      active = false;
-    }
-  }
-  // Warp-aggregated increment: one atomic per distinct cell in the warp.
-  unsigned mask = __ballot_sync(0xffffffffu, active);
-  if (active) {
-    unsigned peers = __match_any_sync(mask, c);
-    int leader = __ffs(peers) - 1;
-    if ((int)(threadIdx.x & 31) == leader) atomicAdd(&cell_count[c], __popc(peers));
-  }
 }
 
 // Places each bond into its cell's range; decrements the counts back to
@@ -220,6 +192,7 @@ __global__ void k_pair_emit(SysConst k, DevState d, int nb, const int *key,
   for (int i = 0; i < m - 1; ++i)
     for (int j = i + 1; j < m; ++j) emit(it[i], it[j]);
   int s0[13], s1[13];
+  unsigned busy = 0;  // the non-empty neighbours: only these are visited
 #pragma unroll
   for (int kk = 0; kk < 13; ++kk) {  // all ranges loaded together
     s0[kk] = s1[kk] = 0;
@@ -230,47 +203,57 @@ __global__ void k_pair_emit(SysConst k, DevState d, int nb, const int *key,
     }
   }
 #pragma unroll
-  for (int kk = 0; kk < 13; ++kk)
+  for (int kk = 0; kk < 13; ++kk) busy |= s0[kk] < s1[kk] ? 1u << kk : 0u;
+  while (busy) {
+    const int kk = __ffs(busy) - 1;
+    busy &= busy - 1;
+    int lo = 0, hi = 0;
+#pragma unroll
+    for (int q2 = 0; q2 < 13; ++q2)
+      if (q2 == kk) {
+        lo = s0[q2];
+        hi = s1[q2];
+      }
     for (int i = 0; i < m; ++i)
-      for (int j = s0[kk]; j < s1[kk]; ++j) emit(it[i], sorted[j]);
+      for (int j = lo; j < hi; ++j) emit(it[i], sorted[j]);
+  }
 }
 
-// Per-bond entry ranges of the rebuilt systems, inside their slot segments,
-// from the exclusive scan of the degrees over all bonds.
-__global__ void k_csr_offsets(DevState d, const int *deg_off, const int *deg) {
-  grid_dep_sync();
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.nb) return;
-  const int r = rep_of_bond(d, b);
-  if (!d.due[r]) return;
-  const ReplicaConst &R = d.rep[r];
-  d.e_off[b] = 2 * R.p0 + (deg_off[b] - deg_off[R.b0]);
-  d.e_cnt[b] = deg[b];
+// First entry slot of bond b, inside its system's slot segment, from the
+// exclusive scan of the degrees over all bonds.
+__device__ __forceinline__ int csr_first(const DevState &d, const ReplicaConst &R,
+                                         const int *deg_off, int b) {
+  return 2 * R.p0 + (deg_off[b] - deg_off[R.b0]);
 }
 
 // Entries (pair << 1 | role) of every bond of the rebuilt systems; role 0 =
 // obj1, 1 = obj2.  The degree array is decremented back to zero.
-__global__ void k_csr_fill(DevState d, int *deg) {
+__global__ void k_csr_fill(DevState d, int *deg, const int *deg_off) {
   grid_dep_sync();
   int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= d.pcap_total) return;
   int r;
   if (!pair_live(d, p, r) || !d.due[r]) return;
+  const ReplicaConst &R = d.rep[r];
   int a = d.pa[p], b = d.pb[p];
   int sa = atomicSub(&deg[a], 1) - 1;
   int sb = atomicSub(&deg[b], 1) - 1;
-  d.e_ent[d.e_off[a] + sa] = p << 1;
-  d.e_ent[d.e_off[b] + sb] = (p << 1) | 1;
+  d.e_ent[csr_first(d, R, deg_off, a) + sa] = p << 1;
+  d.e_ent[csr_first(d, R, deg_off, b) + sb] = (p << 1) | 1;
 }
 
 // Sorts each bond's entries by pair index = the order in which the
 // reference's serial ApplyPairInteractions adds them to the bond, then
-// records the slot of each (pair, role) entry.
-__global__ void k_csr_sort_pos(DevState d) {
+// records the slot of each (pair, role) entry and the bond's entry range.
+__global__ void k_csr_sort_pos(DevState d, const int *deg_off) {
   grid_dep_sync();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= d.nb || !d.due[rep_of_bond(d, b)]) return;
-  int e0 = d.e_off[b], e1 = e0 + d.e_cnt[b];
+  if (b >= d.nb) return;
+  const int r = rep_of_bond(d, b);
+  if (!d.due[r]) return;
+  const int e0 = csr_first(d, d.rep[r], deg_off, b), e1 = e0 + deg_off[b + 1] - deg_off[b];
+  d.e_off[b] = e0;
+  d.e_cnt[b] = e1 - e0;
   int *e = d.e_ent;
   for (int i = e0 + 1; i < e1; ++i) {
     int v = e[i], j = i - 1;
@@ -1231,8 +1214,55 @@ template int launch_soa_to_aos<double>(int, const double *, const double *, cons
 
 // Exclusive scan in[0..n) -> out[0..n], out[n] = total.  tmp holds
 // scan_temp_ints(n) ints.  Returns launches issued.
+// The whole scan in one block, for at most kScanOne elements: one launch
+// instead of two, which is what a scan this small costs (2,000 bonds: 2.3 us
+// against 4.4).
+constexpr int kScanOne = 8192;
+
+__global__ void __launch_bounds__(1024) k_scan_one(const int *in, int *out, int n) {
+  grid_dep_sync();
+  __shared__ int warp_sum[32];
+  constexpr int ITEMS = kScanOne / 1024;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, base = threadIdx.x * ITEMS;
+  int v[ITEMS], sum = 0;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    v[i] = base + i < n ? in[base + i] : 0;
+    sum += v[i];
+  }
+  int x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sum[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int s = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += y;
+    }
+    warp_sum[lane] = s;
+  }
+  __syncthreads();
+  int run = x - sum + (w > 0 ? warp_sum[w - 1] : 0);
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    if (base + i < n) out[base + i] = run;
+    run += v[i];
+  }
+  if (threadIdx.x == 0) out[n] = warp_sum[31];
+}
+
 int launch_exclusive_scan(const int *in, int *out, long long n, int *tmp, cudaStream_t st,
                           unsigned *occ) {
+  if (n <= kScanOne && !occ) {
+    launch_pdl(k_scan_one, dim3(1), dim3(1024), 0, st, in, out, (int)n);
+    return 1;
+  }
   int tiles = cdiv(n, SCAN_TILE);
   if (tiles == 0) tiles = 1;
   const bool vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
@@ -1244,13 +1274,6 @@ int launch_exclusive_scan(const int *in, int *out, long long n, int *tmp, cudaSt
     launch_pdl(k_scan_down<false>, dim3(tiles), dim3(SCAN_BLOCK), 0, st, in, out, (int)n, tmp, occ);
   }
   return 2;
-}
-
-int launch_bin_count(const SysConst &k, const DevState &d, int *key,
-                     int *cell_count, cudaStream_t st) {
-  if (k.n_dim == 3) launch_pdl(k_bin_count<3>, dim3(cdiv(d.nb, 256)), dim3(256), 0, st, k, d, key, cell_count);
-  else launch_pdl(k_bin_count<2>, dim3(cdiv(d.nb, 256)), dim3(256), 0, st, k, d, key, cell_count);
-  return 1;
 }
 
 int launch_bond_cells(const SysConst &k, const DevState &d, int *xyz,
@@ -1284,10 +1307,10 @@ int launch_pair_emit(const SysConst &k, const DevState &d, const int *key,
 }
 
 int launch_csr(const DevState &d, int *deg, const int *deg_off, cudaStream_t st) {
-  launch_pdl(k_csr_offsets, dim3(cdiv(d.nb, 256)), dim3(256), 0, st, d, deg_off, deg);
-  launch_pdl(k_csr_fill, dim3(cdiv(d.pcap_total > 0 ? d.pcap_total : 1, 256)), dim3(256), 0, st, d, deg);
-  launch_pdl(k_csr_sort_pos, dim3(cdiv(d.nb, 256)), dim3(256), 0, st, d);
-  return 3;
+  launch_pdl(k_csr_fill, dim3(cdiv(d.pcap_total > 0 ? d.pcap_total : 1, 256)), dim3(256), 0, st, d,
+             deg, deg_off);
+  launch_pdl(k_csr_sort_pos, dim3(cdiv(d.nb, 256)), dim3(256), 0, st, d, deg_off);
+  return 2;
 }
 
 // ---------------------------------------------------------------------------

@@ -41,8 +41,6 @@ int launch_soa_to_aos(int n, const T *x, const T *y, const T *z, double *aos, cu
 // With occ, also one bit per element (set where it is non-zero), 32 to a word.
 int launch_exclusive_scan(const int *in, int *out, long long n, int *tmp,
                           cudaStream_t st, unsigned *occ = nullptr);
-int launch_bin_count(const SysConst &k, const DevState &d, int *key,
-                     int *cell_count, cudaStream_t st);
 int launch_bond_cells(const SysConst &k, const DevState &d, int *xyz,
                       cudaStream_t st);
 // The rebuild pass covers the systems flagged in d.due; bonds of other
