@@ -122,3 +122,32 @@ def test_packed_units_keep_systems_apart(precision):
         ctx.close()
     assert np.array_equal(both.sites(), np.concatenate(alone))
     both.close()
+
+
+@pytest.mark.parametrize("n_fil", [3, 12, 70])
+def test_long_pair_lists_bitwise(n_fil):
+    """Bundles whose bonds have up to about 10, 40 and 230 pairs: the entries
+    of a bond are sorted by its thread, by its warp, or in memory, and its
+    forces are added in pair order."""
+    import simcore_b200 as sc
+    from checkers import Oracle
+    rng = np.random.default_rng(n_fil)
+    sites = []
+    for i in range(n_fil):
+        head = np.array([0.013 * i, 0.4 * rng.random(), 0.0])
+        sites.append(head + np.arange(6)[:, None] * np.array([0.0, 0.0, 1.0]))
+    fils = [dict(length=5.0 * (1 + 1e-12), persistence_length=100.0, diameter=1.0,
+                 min_bond_length=0.666, friction_ratio=2.0)] * n_fil
+    system = dict(n_dim=3, system_radius=12.0, delta=1e-7, seed=1)
+    ctx = sc.Context(system, fils, np.concatenate(sites), precision="fp64")
+    oracle = Oracle(system, fils, np.concatenate(sites))
+    ctx.step(2)
+    oracle.step(2)
+    most = np.bincount(ctx.pairs().ravel()).max()
+    assert most > {3: 2, 12: 16, 70: 128}[n_fil]
+    assert np.array_equal(ctx.pairs(), oracle.pairs())
+    for got, want in zip(ctx.bond_forces(), oracle.bond_forces()):
+        assert np.array_equal(got, want)
+    assert np.array_equal(ctx.sites(), oracle.sites())
+    ctx.close()
+    oracle.close()
