@@ -1709,12 +1709,13 @@ int launch_integrate(const SysConst &k, const DevState &d, int nblocks, int C,
     ++launched;
   }
   if (nblocks == 0) return launched;
+  const int beside = launched;  // after the team kernel
   size_t smem = integrate_smem_bytes(C, d.blk_maxf);
 #define SC_INTEGRATE(ND, P, MC)                                                                  \
   ((C == MC) ? launch_pdl(k_integrate<ND, P, false, MC, false, true>, dim3(nblocks), dim3(C), smem, \
-                          st, k, d, midstep, rbuf, interaction, capture)                        \
+                          st, k, d, midstep, rbuf, interaction, capture, beside)                \
              : launch_pdl(k_integrate<ND, P, false, MC>, dim3(nblocks), dim3(C), smem, st, k, d,  \
-                          midstep, rbuf, interaction, capture))
+                          midstep, rbuf, interaction, capture, beside))
   if (C <= 128) {
     if (k.n_dim == 3) {
       if (prec == 0) SC_INTEGRATE(3, 0, 128); else SC_INTEGRATE(3, 1, 128);
