@@ -41,8 +41,11 @@ __device__ __forceinline__ void grid_dep_sync() {
 // The same in two parts, for a kernel that runs beside the one before it: that
 // one's wait is enough for its own reads (it lets this one launch only after
 // it), it writes nothing that this one reads, and this one waits for it last,
-// so that whoever waits for this one has waited for both.
-__device__ __forceinline__ void grid_dep_launch() {
+// so that whoever waits for this one has waited for both.  The fence keeps
+// this kernel's reads from being served from before it started (an L1 line
+// of an earlier kernel on the same SM): no wait of its own orders them.
+__device__ __forceinline__ void grid_dep_beside() {
+  __threadfence();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void grid_dep_wait() {

@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // writes every load below reads: wait for it first.
   // (beside: launched right after the team kernel of the same step, whose
   // filaments are others; it has waited for what this one reads.)
-  if (beside) grid_dep_launch();
+  if (beside) grid_dep_beside();
   else if (FUSE || !interaction) grid_dep_sync();
   // A rebuild of this step whose list outgrew its segment stops the step
   // before its first store (uniform over the grid: nothing in this kernel
