@@ -1659,8 +1659,11 @@ static void set_attr(size_t smem) {
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
+// The limit is the instantiation's own largest block, not this context's: a
+// second context with smaller blocks must not lower it under the first's.
 void prepare_integrate(int C) {
-  size_t smem = integrate_smem_bytes(C, C / 2);
+  const int most = C <= 128 ? 128 : C <= 192 ? 192 : C <= 256 ? 256 : 512;
+  size_t smem = integrate_smem_bytes(most, most / 2);
   if (C <= 128) {
     set_attr<3, 0, 128>(smem);
     set_attr<3, 1, 128>(smem);
@@ -1682,7 +1685,7 @@ void prepare_integrate(int C) {
     set_attr<2, 0, 512>(smem);
     set_attr<2, 1, 512>(smem);
   }
-  prepare_integrate_fast(C);
+  prepare_integrate_fast(C, smem);
 }
 
 int launch_integrate(const SysConst &k, const DevState &d, int nblocks, int C,

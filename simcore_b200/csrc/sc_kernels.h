@@ -143,7 +143,7 @@ void prepare_integrate(int C);
 int launch_integrate(const SysConst &k, const DevState &d, int nblocks, int C,
                      int midstep, int rbuf, int interaction, int capture,
                      int prec, bool fast, cudaStream_t st, bool fuse = false);
-void prepare_integrate_fast(int C);
+void prepare_integrate_fast(int C, size_t smem);
 int launch_integrate_fast(const SysConst &k, const DevState &d, int nblocks, int C,
                           int midstep, int rbuf, int interaction, int capture,
                           cudaStream_t st, bool fuse);

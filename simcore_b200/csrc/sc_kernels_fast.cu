@@ -40,8 +40,7 @@ static void launch_block_fast(const SysConst &k, const DevState &d, int nblocks,
                midstep, rbuf, interaction, capture, beside);
 }
 
-void prepare_integrate_fast(int C) {
-  size_t smem = integrate_smem_bytes(C, C / 2);
+void prepare_integrate_fast(int C, size_t smem) {
   if (C <= 128) {
     set_attr_fast<3, 128>(smem);
     set_attr_fast<2, 128>(smem);

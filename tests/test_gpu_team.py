@@ -151,3 +151,25 @@ def test_long_pair_lists_bitwise(n_fil):
     assert np.array_equal(ctx.sites(), oracle.sites())
     ctx.close()
     oracle.close()
+
+
+@pytest.mark.parametrize("blocks", [(256, 224), (128, 96)])
+def test_layouts_of_two_contexts(blocks):
+    """Contexts with different block sizes share compiled kernels; the second
+    one's smaller shared memory does not become the first one's limit."""
+    import simcore_b200 as sc
+    from checkers import Oracle
+    # Two-bond filaments: as much shared memory a block as its size allows.
+    system, fils, sites = _lattice(3, np.array([2] * 400), 60.0, seed=9, min_bond_length=2.0)
+    ctxs = []
+    for size in blocks:
+        ctxs.append(sc.Context(system, fils, sites, precision="fp64"))
+        ctxs[-1].set_integrator_layout(0, size)
+    oracle = Oracle(system, fils, sites)
+    oracle.step(4)
+    for ctx in ctxs:
+        ctx.step_graph(4)
+        assert np.array_equal(ctx.sites(), oracle.sites())
+    for ctx in ctxs:
+        ctx.close()
+    oracle.close()
