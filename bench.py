@@ -673,7 +673,7 @@ def run_reference(args, rank, world):
 
 def layout_sweep(args):
     """--layout-sweep: for both precisions and every integrator layout that
-    holds the workload (warp kernel on or off, blocks of 64-256 sites), the
+    holds the workload (team kernel on or off, blocks of 64-256 sites), the
     CUDA-event time of the pair and integrator kernels of a host-driven
     reference step (L2 warm) and of a captured 20-step launch (L2 flushed
     first); one JSON line per layout.  Layouts are what sc_autotune chooses

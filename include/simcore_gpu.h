@@ -289,9 +289,9 @@ sc_status sc_get_bond_geometry(sc_ctx *ctx, double *pos, double *spos,
  * effect in SC_PREC_FP64, which is always exact. */
 sc_status sc_set_fast_integrator(sc_ctx *ctx, int on);
 /* Integrator layout, a tuning knob (every layout gives the same results):
- * filaments of at most warp_max_sites sites (<= 32) run on the
- * warp-synchronous kernel, one warp per group of whole filaments; longer
- * ones on the block kernel, block_sites sites per block (a multiple of 32 up
+ * filaments of at most warp_max_sites sites (<= 32) run on the team
+ * kernel, a team of one warp's lanes per filament; longer ones on the block
+ * kernel, block_sites sites per block (a multiple of 32 up
  * to 512, at least the longest such filament; 0 picks 128, 256 or 512).
  * warp_max_sites 0 puts every filament on the block kernel. */
 sc_status sc_set_integrator_layout(sc_ctx *ctx, int warp_max_sites, int block_sites);

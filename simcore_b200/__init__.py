@@ -220,8 +220,8 @@ class Context:
         self._check(lib.sc_set_fast_integrator(self.h, ctypes.c_int(1 if on else 0)))
 
     def set_integrator_layout(self, warp_max_sites=32, block_sites=0):
-        """Filaments of at most warp_max_sites sites on the warp-synchronous
-        integrator (0: none), the rest on blocks of block_sites sites."""
+        """Filaments of at most warp_max_sites sites on the team integrator
+        (one warp's lanes per filament; 0: none), the rest on blocks of block_sites sites."""
         self._check(lib.sc_set_integrator_layout(self.h, ctypes.c_int(warp_max_sites),
                                                  ctypes.c_int(block_sites)))
 

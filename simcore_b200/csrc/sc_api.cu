@@ -514,6 +514,9 @@ sc_status layout_integrator(sc_ctx *c) {
                         (const void *)d.blk_ns, (const void *)d.blk_list, (const void *)d.blk_slot,
                         (const void *)d.tm_lane})
     dfree(c, const_cast<void *>(q));
+  d.blk_site0 = d.blk_f0 = d.blk_nf = d.blk_ns = nullptr;  // (an upload below may fail)
+  d.blk_list = nullptr;
+  d.blk_slot = d.tm_lane = nullptr;
   auto up = [&](auto **dst, const auto &v) -> sc_status {
     using T = typename std::remove_reference<decltype(v)>::type::value_type;
     T *q = nullptr;
@@ -524,8 +527,6 @@ sc_status layout_integrator(sc_ctx *c) {
     *dst = q;
     return SC_OK;
   };
-  d.blk_list = nullptr;
-  d.blk_slot = nullptr;
   CKS(up(&d.blk_site0, blk_site0));
   CKS(up(&d.blk_f0, blk_f0));
   CKS(up(&d.blk_nf, blk_nf));

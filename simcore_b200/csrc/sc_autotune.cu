@@ -1,4 +1,4 @@
-// Integrator work layout (warp kernel for short filaments, block size of the
+// Integrator work layout (team kernel for short filaments, block size of the
 // block kernel) and its autotuner, cached per shape.
 #include "sc_context.h"
 
@@ -23,7 +23,7 @@ sc_status sc_set_integrator_layout(sc_ctx *c, int warp_max_sites, int block_site
   return st;
 }
 
-// Autotuner.  Candidate integrator layouts (warp kernel or not, block size)
+// Autotuner.  Candidate integrator layouts (team kernel or not, block size)
 // and pair-kernel block sizes (128 or 256 threads) are timed on the
 // context's own state: the arrays they write are saved first and restored
 // afterwards, so the simulation is unchanged.  The fastest choices are
@@ -78,7 +78,7 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
     }
   }
   // Candidates: every block size that holds the longest block-kernel
-  // filament, with and without the warp kernel for filaments of <= 32 sites.
+  // filament, with and without the team kernel for filaments of <= 32 sites.
   std::vector<std::pair<int, int>> cand;
   for (int w : {32, 0}) {
     if (w == 32 && min_n > 32) continue;
