@@ -683,7 +683,9 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // Grid-stride over the pair slots, so a captured launch stays correct
 // whatever length the lists grow to between captures.  A single system's
 // list is the prefix of its segment; with several systems every slot checks
-// that it holds a current pair of its system.
+// that it holds a current pair of its system.  A list that outgrew its segment
+// (the step stops, its rebuild is redone) has holes, whose entries nothing has
+// written: it is not evaluated.
 // NPX (mixed only): nearly parallel pairs are evaluated in FP64
 // (eval_near_parallel) by the thread that meets them.
 // The list and its slot indices date from the last rebuild, whose kernels
@@ -695,7 +697,7 @@ __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
     k_pair_eval(SysConst k, DevState d, int rbuf) {
   if (d.nrep == 1) {
     const ReplicaConst &R = d.rep[0];
-    const int np = min(d.np_rep[0], R.pcap);
+    const int np = d.np_rep[0] <= R.pcap ? d.np_rep[0] : 0;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     PairIdx ix = {0, 0, 0, 0};
     if (p < np) ix = pair_idx(d, p);
@@ -717,7 +719,8 @@ __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.pcap_total;
        p += gridDim.x * blockDim.x) {
     int r;
-    if (pair_live(d, p, r) && !pair_eval_one<ND, PREC, NPX>(k, d, d.rep[r], rbuf, p, pair_idx(d, p)))
+    if (pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap &&
+        !pair_eval_one<ND, PREC, NPX>(k, d, d.rep[r], rbuf, p, pair_idx(d, p)))
       if (NPX) near_parallel_fp64<ND>(k, d, d.rep[r], p);
   }
 }
