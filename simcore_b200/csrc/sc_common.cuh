@@ -59,8 +59,11 @@ enum : unsigned {
   ST_UNPHYSICAL = 4u,     // accumulated displacement above 10000
   ST_BAD_CELL = 8u,       // cell index out of range (non-finite position)
   ST_BAD_INPUT = 16u,     // caller's device data out of range (site offsets)
-  ST_TETHER = 32u         // a crosslink anchor left the bonds it can sit on
+  ST_TETHER = 32u,        // a crosslink anchor left the bonds it can sit on
+  ST_STOP = 64u           // a chained run stopped after an error (never left set)
 };
+// The steps that are already launched do nothing.
+constexpr unsigned ST_HALT = ST_LIST_OVERFLOW | ST_STOP;
 
 // Bond geometry for the FP64 pair stage: the reference's Bond state after
 // Bond::ReInit (scaled position, unit orientation, length).  64 bytes.

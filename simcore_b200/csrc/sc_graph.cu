@@ -1,10 +1,67 @@
-// sc_step_graph: the reference step loop captured as one CUDA graph, a WHILE
-// loop of Brownian-dynamics steps with device-decided rebuilds.
+// sc_step_graph: the reference step loop without host round trips, rebuilds
+// decided on the device: captured as one CUDA graph, a WHILE loop of
+// Brownian-dynamics steps, or, of small contexts, launched as a chain.
 #include "sc_context.h"
+
+#include <optional>
 
 using namespace scapi;
 
+// Contexts whose steps are chained (enqueue_chain) instead of looped in a
+// graph.  Per BD step, chain against graph: 2,000 bonds 34.7 us against 40.9
+// (FP64) and 24.1 against 30.5 (mixed), 12,000 bonds 38.1 and 39.6, 29.3 and
+// 31.8, 16,000 bonds the same; beyond, one cluster's rebuild (125 us at 20,000
+// bonds) costs more than the loop's conditional nodes.  The cluster also scans
+// one counter per 32 cells; the suspensions of these sizes have up to 11,000.
+static const int kChainBonds = 12288;
+static const int kChainGroups = 32768;
+
 extern "C" {
+
+// The launches of one BD step after its rebuild decision.
+static int bd_step(sc_ctx *c, bool fuse, bool chain) {
+  const int interaction = c->desc.interaction_flag ? 1 : 0;
+  int n = 0;
+  for (int half = 0; half < 2; ++half) {
+    const int rb = half == 0 ? c->rbuf : 1 - c->rbuf;
+    // A graph body's first kernel follows a conditional rebuild node (or the
+    // body's start), not a kernel: it is launched without the programmatic
+    // attribute.  A chained step's follows the control kernel, which may write
+    // the pair list: the pair kernel then waits first.
+    // The second half is the even (full) step: crosslink tethers first.
+    if (half == 1 && interaction) n += sc::launch_tether(c->k, c->d, c->st);
+    if (interaction && !fuse) {
+      std::optional<sc::PdlOff> alone;
+      if (half == 0 && !chain) alone.emplace();
+      n += sc::launch_pairs(c->k, c->d, rb, c->prec, (int)(c->np + c->np / 8), c->st, c->npx,
+                            c->pair_block, half == 0 && chain);
+    }
+    if (interaction && c->k.thermo) n += sc::launch_thermo(c->k, c->d, c->prec, c->st);
+    if (half == 0 && (!interaction || fuse)) {
+      sc::PdlOff off;
+      n += sc::launch_integrate(c->k, c->d, c->nblocks, c->C, 1, rb, interaction, c->capture, c->prec,
+                           c->fast, c->st, fuse);
+    } else {
+      n += sc::launch_integrate(c->k, c->d, c->nblocks, c->C, half == 0 ? 1 : 0, rb, interaction,
+                           c->capture, c->prec, c->fast, c->st, fuse);
+    }
+  }
+  return n;
+}
+
+// Steps launched one after another with a control kernel between them, for
+// small contexts: no conditional nodes.
+static void enqueue_chain(sc_ctx *c, int bd) {
+  const bool fuse = fused_pairs(c);
+  const int stoch = c->desc.stoch_flag ? 1 : 0;
+  c->graph_fused = fuse;
+  for (int i = 0; i <= bd; ++i) {
+    c->launches += sc::launch_step_control(c->k, c->d, c->rb, c->prec, stoch, i == 0 ? bd : 0,
+                                           i > 0, i < bd, host_report(c), c->st);
+    if (i < bd) c->launches += bd_step(c, fuse, true);
+  }
+  c->launches += sc::launch_report(c->d, host_report(c), 1, c->st);
+}
 
 // Captures one graph: head (loop condition, first rebuild decision) ->
 // WHILE (loop_count > 0) { IF(rebuild) -> midstep -> full step -> tail (next
@@ -59,33 +116,7 @@ static sc_status build_graph(sc_ctx *c) {
                                    tail.size(), cudaStreamCaptureModeRelaxed));
   const bool fuse = fused_pairs(c);
   c->graph_fused = fuse;
-  for (int half = 0; half < 2; ++half) {
-    const int rb = half == 0 ? c->rbuf : 1 - c->rbuf;
-    // The body's first kernel follows the conditional rebuild node (or the
-    // body's start), not a kernel: it is launched without the programmatic
-    // attribute.
-    // The second half is the even (full) step: crosslink tethers first.
-    if (half == 1 && interaction) sc::launch_tether(c->k, c->d, c->st);
-    if (interaction && !fuse) {
-      if (half == 0) {
-        sc::PdlOff off;
-        sc::launch_pairs(c->k, c->d, rb, c->prec, (int)(c->np + c->np / 8), c->st, c->npx,
-                         c->pair_block);
-      } else {
-        sc::launch_pairs(c->k, c->d, rb, c->prec, (int)(c->np + c->np / 8), c->st, c->npx,
-                         c->pair_block);
-      }
-    }
-    if (interaction && c->k.thermo) sc::launch_thermo(c->k, c->d, c->prec, c->st);
-    if (half == 0 && (!interaction || fuse)) {
-      sc::PdlOff off;
-      sc::launch_integrate(c->k, c->d, c->nblocks, c->C, 1, rb, interaction, c->capture, c->prec,
-                           c->fast, c->st, fuse);
-    } else {
-      sc::launch_integrate(c->k, c->d, c->nblocks, c->C, half == 0 ? 1 : 0, rb, interaction,
-                           c->capture, c->prec, c->fast, c->st, fuse);
-    }
-  }
+  bd_step(c, fuse, false);
   sc::launch_loop_tail(c->d, c->desc.stoch_flag ? 1 : 0, h_loop, h_if, interaction, c->st);
   CK(cudaStreamEndCapture(c->st, &body));
   // What the host reads afterwards.
@@ -128,13 +159,20 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
     // rebuild is redone host-side and the run resumes with that step.
     for (int attempt = 0; bd > 0; ++attempt) {
       if (attempt == 8) return fail(c, SC_ERR_LIST_OVERFLOW, "pair list kept overflowing inside captured runs");
-      if (!c->graph_exec || c->graph_rbuf != c->rbuf) CKS(build_graph(c));
+      const bool chain = c->desc.interaction_flag && c->nb <= kChainBonds &&
+                         c->rb.n_groups <= kChainGroups;
+      if (!chain && (!c->graph_exec || c->graph_rbuf != c->rbuf)) CKS(build_graph(c));
       // The head reads the step count and the last node writes everything
       // the host looks at, both in pinned memory: no copies, one
       // synchronisation per launch.
       *c->h_loop = bd;
       CK(cudaEventRecord(c->gev0, c->st));
-      CK(cudaGraphLaunch(c->graph_exec, c->st));
+      if (chain) {
+        enqueue_chain(c, bd);
+        CK(cudaGetLastError());
+      } else {
+        CK(cudaGraphLaunch(c->graph_exec, c->st));
+      }
       CK(cudaEventRecord(c->gev1, c->st));
       c->pairs_ready = false;
       CK(cudaStreamSynchronize(c->st));
@@ -163,8 +201,9 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
               ? 1 + (c->d.nx ? 2 : 0) +
                     2 * ((c->graph_fused ? 0 : 1) + int_l + (c->k.thermo ? 1 : 0))
               : 1 + 2 * int_l;
-      c->launches += 2 + (long long)(done + (overflow ? 1 : 0)) * per_bd +
-                     (nr1 - nr0) * c->rebuild_kernels;
+      if (!chain)
+        c->launches += 2 + (long long)(done + (overflow ? 1 : 0)) * per_bd +
+                       (nr1 - nr0) * c->rebuild_kernels;
       bd -= done;
       if (!overflow) {
         CKS(check_status(c));  // status and maxima were read with the counters

@@ -694,7 +694,8 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // wait; the bond geometry, which that kernel may be writing, after it.
 template <int ND, int PREC, bool NPX, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
-    k_pair_eval(SysConst k, DevState d, int rbuf) {
+    k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first) {
+  if (wait_first) grid_dep_sync();
   if (d.nrep == 1) {
     const ReplicaConst &R = d.rep[0];
     const int np = d.np_rep[0] <= R.pcap ? d.np_rep[0] : 0;
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(128) k_tether(SysConst k, DevState d) {
   const int A = blockIdx.x * blockDim.x + threadIdx.x, a = A & 1;  // the anchor; link A / 2
   const unsigned lanes = __ballot_sync(0xffffffffu, A < 2 * d.nx);
   if (A >= 2 * d.nx) return;  // pairs of lanes together
-  if (*d.status & ST_LIST_OVERFLOW) return;  // the step stopped at its rebuild
+  if (*d.status & ST_HALT) return;  // the step stopped at its rebuild
   const int f = d.xl_fil[A];
   const FilConst &fc = d.fil[f];
   const int nbf = fc.n - 1, b0 = fc.site0 - f;
@@ -1427,26 +1428,34 @@ int launch_zero_dr(const DevState &d, cudaStream_t st) {
 
 template <int BLOCK>
 static void launch_pairs_block(const SysConst &k, const DevState &d, int rbuf, int prec, int grid,
-                               cudaStream_t st, bool npx) {
+                               cudaStream_t st, bool npx, int wait_first) {
   if (k.n_dim == 3) {
-    if (prec == 0) launch_pdl(k_pair_eval<3, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
-    else if (!npx) launch_pdl(k_pair_eval<3, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
-    else launch_pdl(k_pair_eval<3, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
+    if (prec == 0) launch_pdl(k_pair_eval<3, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                              wait_first);
+    else if (!npx) launch_pdl(k_pair_eval<3, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                             wait_first);
+    else launch_pdl(k_pair_eval<3, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                    wait_first);
   } else {
-    if (prec == 0) launch_pdl(k_pair_eval<2, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
-    else if (!npx) launch_pdl(k_pair_eval<2, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
-    else launch_pdl(k_pair_eval<2, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf);
+    if (prec == 0) launch_pdl(k_pair_eval<2, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                              wait_first);
+    else if (!npx) launch_pdl(k_pair_eval<2, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                             wait_first);
+    else launch_pdl(k_pair_eval<2, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
+                    wait_first);
   }
 }
 
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
-                 int expected, cudaStream_t st, bool npx, int block) {
+                 int expected, cudaStream_t st, bool npx, int block, bool wait_first) {
   if (d.nrep > 1) expected = d.pcap_total;
   npx = npx && prec != 0;
   if (block == 128)
-    launch_pairs_block<128>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 128), st, npx);
+    launch_pairs_block<128>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 128), st, npx,
+                            wait_first);
   else
-    launch_pairs_block<256>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 256), st, npx);
+    launch_pairs_block<256>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 256), st, npx,
+                            wait_first);
   return 1;
 }
 
@@ -1470,7 +1479,7 @@ int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
 template <int ND, int PREC>
 __global__ void __launch_bounds__(256) k_thermo(SysConst k, DevState d) {
   grid_dep_sync();
-  if (*d.status & ST_LIST_OVERFLOW) return;  // the step stopped at its rebuild
+  if (*d.status & ST_HALT) return;  // the step stopped at its rebuild
   const int r = blockIdx.y;
   const ReplicaConst &R = d.rep[r];
   const int np = min(d.np_rep[r], R.pcap);

@@ -105,6 +105,11 @@ struct HostReport {
   unsigned long long *dr;  // per system: displacement maximum
   int *np;                 // per system: pairs
 };
+// Between two BD steps of a chained run (no conditional graph nodes): ends the
+// step before (close), decides and does the next one's rebuild (more).
+int launch_step_control(const SysConst &k, const DevState &d, const RebuildBufs &rb, int prec,
+                        int stoch, int first, int close, int more, const HostReport &out,
+                        cudaStream_t st);
 // graph: also the loop's remaining steps and the rebuild passes, for a captured
 // run's end.
 int launch_report(const DevState &d, const HostReport &out, int graph, cudaStream_t st);
@@ -124,9 +129,11 @@ int launch_zero_dr(const DevState &d, cudaStream_t st);
 // sites, in place.  The kernel loads the pair list and slot indices before
 // it waits on the kernel launched just before it (programmatic dependent
 // launch): that kernel must not write them -- the last kernel of a rebuild
-// does not -- or the launch must be made without the overlap (PdlOff).
+// does not -- or the launch must be made without the overlap (PdlOff), or with
+// wait_first: the kernel waits before it loads anything.
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
-                 int expected, cudaStream_t st, bool npx = false, int block = 256);
+                 int expected, cudaStream_t st, bool npx = false, int block = 256,
+                 bool wait_first = false);
 // Crosslink tethers of an even step into the per-anchor contributions.
 int launch_tether(const SysConst &k, const DevState &d, cudaStream_t st);
 // Thermo: one step's pair virial per system, the pressure record every

@@ -24,6 +24,7 @@
 //   k_rb_place     candidates to their list slots, stored forces zeroed,
 //                  per-bond entries (pair << 1 | role)
 //   k_rb_csr_sort  entries in pair order, slots of both roles, ranges
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "sc_cells.cuh"
@@ -44,11 +45,8 @@ namespace sc {
 // Bound by memory latency: 71,758 filaments in 64 systems took 40 us with
 // three dependent lookups a site for its system and every thread walking the
 // systems one after another for their words, 8.9 us now.
-template <int ND>
-__global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, RebuildBufs rb) {
-  grid_dep_sync();
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nthreads = gridDim.x * blockDim.x;
+__device__ __forceinline__ void rb_systems(const DevState &d, const RebuildBufs &rb, int tid,
+                                           int nthreads) {
   if (tid == 0) {
     *d.n_rebuilds += 1;
     *rb.cand_n = 0;
@@ -60,7 +58,12 @@ __global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, Rebuild
   }
   for (int w = tid; w < rb.n_groups; w += nthreads)
     if (d.nrep == 1 || d.due[rb.grp_rep[w]]) rb.occ[w] = 0u;
-  const int b = tid;
+}
+
+// (A whole warp's consecutive bonds; those past the last do nothing.)
+template <int ND>
+__device__ __forceinline__ void rb_key(const SysConst &k, const DevState &d, const RebuildBufs &rb,
+                                       int b) {
   bool in = false;
   int g = 0;
   if (b < d.nb) {
@@ -98,25 +101,34 @@ __global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, Rebuild
   }
 }
 
+template <int ND>
+__global__ void __launch_bounds__(256) k_rb_keys(SysConst k, DevState d, RebuildBufs rb) {
+  grid_dep_sync();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  rb_systems(d, rb, tid, gridDim.x * blockDim.x);
+  rb_key<ND>(k, d, rb, tid);
+}
+
 // Each rebuilt bond into its group's range of the scanned offsets (any
 // order inside the group); decrements the counts back to zero, ready for
 // the next rebuild.
-__global__ void k_rb_scatter(DevState d, RebuildBufs rb) {
-  grid_dep_sync();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void rb_scatter(const DevState &d, const RebuildBufs &rb, int b) {
   if (b >= d.nb || !d.due[rep_of_bond(d, b)]) return;
   const int g = (int)(rb.key[b] >> 5);
   const int slot = atomicSub(&rb.gcount[g], 1) - 1;
   rb.tmp[rb.gstart[g] + slot] = b;
 }
 
+__global__ void k_rb_scatter(DevState d, RebuildBufs rb) {
+  grid_dep_sync();
+  rb_scatter(d, rb, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // Sorted position of every rebuilt bond: its group's first entry plus the
 // number of bonds of the group that come before it by (cell, bond id).  The
 // first of a cell writes the cell's start and occupancy bit, the last its
 // end.
-__global__ void k_rb_rank(DevState d, RebuildBufs rb) {
-  grid_dep_sync();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void rb_rank(const DevState &d, const RebuildBufs &rb, int q) {
   if (q >= rb.gstart[rb.n_groups]) return;
   const int b = rb.tmp[q];
   const uint32_t c = rb.key[b];
@@ -141,6 +153,11 @@ __global__ void k_rb_rank(DevState d, RebuildBufs rb) {
     atomicOr(&rb.occ[c >> 5], 1u << (c & 31));
   }
   if (last) rb.range[c].y = pos + 1;
+}
+
+__global__ void k_rb_rank(DevState d, RebuildBufs rb) {
+  grid_dep_sync();
+  rb_rank(d, rb, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __device__ __forceinline__ bool occupied(const unsigned *occ, int c) {
@@ -236,11 +253,11 @@ __device__ __forceinline__ void cell_pairs_visit(const SysConst &k, const DevSta
 constexpr int kCountBlock = 128;
 constexpr int kHeadBuf = 8;
 
-__global__ void __launch_bounds__(kCountBlock) k_rb_count(SysConst k, DevState d, RebuildBufs rb) {
-  __shared__ int2 sbuf[kCountBlock][kHeadBuf];
-  __shared__ int swarp[kCountBlock / 32];
-  grid_dep_sync();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+// (A block's consecutive entries; called by all of its BLOCK threads.)
+template <int BLOCK>
+__device__ __forceinline__ void rb_count(const SysConst &k, const DevState &d,
+                                         const RebuildBufs &rb, int q, int2 (*sbuf)[kHeadBuf],
+                                         int *swarp) {
   const int t = threadIdx.x, lane = t & 31;
   int cnt = 0;
   const ReplicaConst *R = nullptr;
@@ -271,14 +288,14 @@ __global__ void __launch_bounds__(kCountBlock) k_rb_count(SysConst k, DevState d
   if (t == 0) {
     int run = 0;
 #pragma unroll
-    for (int w = 0; w < kCountBlock / 32; ++w) {
+    for (int w = 0; w < BLOCK / 32; ++w) {
       const int v = swarp[w];
       swarp[w] = run;
       run += v;
     }
     const int base = run > 0 ? atomicAdd(rb.cand_n, run) : 0;
 #pragma unroll
-    for (int w = 0; w < kCountBlock / 32; ++w) swarp[w] += base;
+    for (int w = 0; w < BLOCK / 32; ++w) swarp[w] += base;
   }
   __syncthreads();
   const int t0 = swarp[t >> 5] + incl - cnt;
@@ -300,6 +317,13 @@ __global__ void __launch_bounds__(kCountBlock) k_rb_count(SysConst k, DevState d
   }
 }
 
+__global__ void __launch_bounds__(kCountBlock) k_rb_count(SysConst k, DevState d, RebuildBufs rb) {
+  __shared__ int2 sbuf[kCountBlock][kHeadBuf];
+  __shared__ int swarp[kCountBlock / 32];
+  grid_dep_sync();
+  rb_count<kCountBlock>(k, d, rb, blockIdx.x * blockDim.x + threadIdx.x, sbuf, swarp);
+}
+
 // First entry slot of bond b (rebuilt system R): its system's slots start at
 // 2 p0, its bonds' entries follow in bond order.
 __device__ __forceinline__ int entry_first(const RebuildBufs &rb, const ReplicaConst &R, int b) {
@@ -314,9 +338,8 @@ __device__ __forceinline__ int entry_first(const RebuildBufs &rb, const ReplicaC
 // system whose list outgrew its segment gets no entries: its step stops on
 // the overflow bit and is redone.  Threads u < nrep record their system's
 // pair count (the count is kept so the host can size the segment).
-__global__ void k_rb_place(DevState d, RebuildBufs rb, int prec) {
-  grid_dep_sync();
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void rb_place(const DevState &d, const RebuildBufs &rb, int prec,
+                                         int u) {
   if (u < d.nrep && d.due[u]) {
     const ReplicaConst &R = d.rep[u];
     const int np = rb.pair_off[sys_hi(rb, R)] - rb.pair_off[sys_lo(rb, R)];
@@ -354,6 +377,11 @@ __global__ void k_rb_place(DevState d, RebuildBufs rb, int prec) {
       d.e_ent[entry_first(rb, R, e.y) + sb] = (g << 1) | 1;
     }
   }
+}
+
+__global__ void k_rb_place(DevState d, RebuildBufs rb, int prec) {
+  grid_dep_sync();
+  rb_place(d, rb, prec, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The wn entries at w0 sorted by the whole warp (`own`: the list's own lane).
@@ -418,9 +446,9 @@ static __device__ __noinline__ void sort_long_list(int *e_ent, int *pos1, int *p
 // bonds, 388,000 pairs, 43 us, 22 us now.)
 constexpr int kRegEntries = 16;
 
-__global__ void k_rb_csr_sort(DevState d, RebuildBufs rb) {
-  grid_dep_sync();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+// (A whole warp's consecutive bonds.)
+__device__ __forceinline__ void rb_csr_sort(const DevState &d, const RebuildBufs &rb, int b) {
+  const int lane = threadIdx.x & 31;
   int e0 = 0, n = 0;
   if (b < d.nb) {
     const int r = rep_of_bond(d, b);
@@ -467,6 +495,159 @@ __global__ void k_rb_csr_sort(DevState d, RebuildBufs rb) {
   }
 }
 
+__global__ void k_rb_csr_sort(DevState d, RebuildBufs rb) {
+  grid_dep_sync();
+  rb_csr_sort(d, rb, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// ---- a chained step's control: bookkeeping, decision, rebuild in one kernel ---
+// A graph's loop pays 9 us a BD step for its conditional nodes, a third of a
+// small system's step.  Small contexts run without them: their steps are
+// launched one after another, and one cluster of blocks between them ends a
+// step, decides the next one's rebuild and does it when due, phase by phase
+// over the hardware's cluster barrier (the kernels above, over all items in
+// turn).  2,000 bonds, 10 BD steps: 320 us with the loop, 256 so.  Idle it is
+// bound by its launch and three dependent round trips to L2 (4 us); a rebuild
+// by the phases' latencies, 36 us at 2,000 bonds (as the ten kernels), 125 at
+// 20,000.  A cluster and not the chip: its barrier needs no waiting loop and
+// no cooperative launch.
+constexpr int kCtlBlocks = 8;  // the portable cluster size
+constexpr int kCtlThreads = 512;
+
+// Exclusive prefix sums of in[0, n) into out[0, n], the total last, by the
+// cluster: a run of entries per block.  tot: kCtlBlocks, part: one per warp.
+static __device__ __noinline__ void cluster_scan(const int *in, int *out, int n, int *tot,
+                                                 int *part) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int tiles = (n + kCtlThreads - 1) / kCtlThreads;
+  const int run = (tiles + kCtlBlocks - 1) / kCtlBlocks * kCtlThreads;
+  const int lo = min(rank * run, n), hi = min(lo + run, n);
+  int sum = 0;
+  for (int i = lo + t; i < hi; i += kCtlThreads) sum += in[i];
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if (lane == 0) part[w] = sum;
+  __syncthreads();
+  if (t < kCtlBlocks) {
+    int all = 0;
+    for (int i = 0; i < kCtlThreads / 32; ++i) all += part[i];
+    cl.map_shared_rank(tot, t)[rank] = all;
+  }
+  cl.sync();
+  int base = 0, total = 0;
+  for (int i = 0; i < kCtlBlocks; ++i) {
+    if (i < rank) base += tot[i];
+    total += tot[i];
+  }
+  if (rank == 0 && t == 0) out[n] = total;
+  for (int i0 = lo; i0 < hi; i0 += kCtlThreads) {
+    const int i = i0 + t;
+    const int v = i < hi ? in[i] : 0;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();  // the last tile's part is read
+    if (lane == 31) part[w] = x;
+    __syncthreads();
+    int before = 0, tile = 0;
+    for (int j = 0; j < kCtlThreads / 32; ++j) {
+      if (j < w) before += part[j];
+      tile += part[j];
+    }
+    if (i < hi) out[i] = base + before + x - v;
+    base += tile;
+  }
+  cl.sync();
+}
+
+// first: the run's BD steps, at its start (else 0).  close: a BD step lies
+// before.  more: another one follows.  A step whose rebuild overflowed its list
+// did nothing past the rebuild and stays counted as remaining; after it, and
+// after a step that recorded an error, the rest of the run does nothing.
+template <int ND>
+__global__ void __cluster_dims__(kCtlBlocks, 1, 1) __launch_bounds__(kCtlThreads)
+    k_step_control(SysConst k, DevState d, RebuildBufs rb, int prec, int stoch, int first,
+                   int close, int more, HostReport out) {
+  namespace cg = cooperative_groups;
+  __shared__ int2 sbuf[kCtlThreads][kHeadBuf];
+  __shared__ int part[kCtlThreads / 32], tot[kCtlBlocks];
+  __shared__ int go;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), t = threadIdx.x;
+  cl.sync();  // every block has started: its shared memory may be written
+  double limit = 0.0;  // (older than the kernel before)
+  if (rank == 0 && t < d.nrep) limit = d.rep[t].dr_update;
+  grid_dep_sync();
+  if (rank == 0) {
+    // The bookkeeping's operands and the first systems' maxima load together.
+    const unsigned status = *d.status;  // the same word for every thread
+    const unsigned long long mcount = *d.mcount;
+    const int left = *d.loop_count;
+    const bool halted = close && (status & ST_HALT), error = close && status != 0u;
+    bool mine = false;
+    unsigned bad = 0u;
+    for (int r = t; r < d.nrep; r += kCtlThreads) {
+      const double dr = __longlong_as_double((long long)d.dr_max_bits[r]);
+      if (r != t) limit = d.rep[r].dr_update;
+      int due = 0;
+      if (dr > 10000.0 || !(dr == dr)) bad = ST_UNPHYSICAL;
+      else due = dr > limit ? 1 : 0;
+      if (!halted) d.due[r] = due;
+      mine = mine || due;
+    }
+    const int any = __syncthreads_or(mine);  // and every thread has read the status
+    if (t < kCtlBlocks) *cl.map_shared_rank(&go, t) = more && !halted && !error && any;
+    if (bad && !halted) atomicOr(d.status, bad);
+    if (t == 0) {
+      if (first) {
+        *d.loop_count = first;
+        out.rebuilds[0] = *d.n_rebuilds;
+      }
+      if (close && !halted) {
+        if (stoch) *d.mcount = mcount + 1ull;
+        *d.loop_count = error ? 0 : left - 1;
+        if (error && more) atomicOr(d.status, ST_STOP);
+      }
+      if (!more) atomicAnd(d.status, ~ST_STOP);
+    }
+  }
+  cl.sync();
+  if (!go) return;  // the same in every block
+  const int step = kCtlBlocks * kCtlThreads, t0 = rank * kCtlThreads;
+  rb_systems(d, rb, t0 + t, step);
+  for (int i = t0; i < d.nb; i += step) rb_key<ND>(k, d, rb, i + t);
+  cl.sync();
+  cluster_scan(rb.gcount, rb.gstart, rb.n_groups, tot, part);
+  for (int i = t0; i < d.nb; i += step) rb_scatter(d, rb, i + t);
+  cl.sync();
+  for (int i = t0; i < d.nb; i += step) rb_rank(d, rb, i + t);
+  cl.sync();
+  for (int i = t0; i < d.nb; i += step) {
+    rb_count<kCtlThreads>(k, d, rb, i + t, sbuf, part);
+    __syncthreads();  // (part is used again)
+  }
+  cl.sync();
+  cluster_scan(rb.pair_count, rb.pair_off, 2 * d.nb, tot, part);
+  const int cand = max(min(*rb.cand_n, rb.cand_cap), d.nrep);
+  for (int i = t0; i < cand; i += step) rb_place(d, rb, prec, i + t);
+  cl.sync();
+  for (int i = t0; i < d.nb; i += step) rb_csr_sort(d, rb, i + t);
+}
+
+int launch_step_control(const SysConst &k, const DevState &d, const RebuildBufs &rb, int prec,
+                        int stoch, int first, int close, int more, const HostReport &out,
+                        cudaStream_t st) {
+  if (k.n_dim == 3)
+    launch_pdl(k_step_control<3>, dim3(kCtlBlocks), dim3(kCtlThreads), 0, st, k, d, rb, prec, stoch,
+               first, close, more, out);
+  else
+    launch_pdl(k_step_control<2>, dim3(kCtlBlocks), dim3(kCtlThreads), 0, st, k, d, rb, prec, stoch,
+               first, close, more, out);
+  return 1;
+}
 
 int launch_rebuild(const SysConst &k, const DevState &d, const RebuildBufs &rb, int prec,
                    cudaStream_t st, bool first_in_graph) {

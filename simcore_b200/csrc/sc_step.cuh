@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // A rebuild of this step whose list outgrew its segment stops the step
   // before its first store (uniform over the grid: nothing in this kernel
   // sets that bit), so the host can grow the list and redo the step.
-  const bool overflowed = (*d.status & ST_LIST_OVERFLOW) != 0u;
+  const bool overflowed = (*d.status & ST_HALT) != 0u;
   const unsigned long long mcount = *d.mcount;
   const int un = d.blk_uni_n;
   int s0, count, f0, nfb;

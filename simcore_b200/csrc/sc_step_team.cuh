@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, K == 1 ? 5 : 4)
   const bool lead = act[0] && j0 == 0;
 
   // ---- every global read of the step, issued together -----------------------
-  const bool overflowed = (*d.status & ST_LIST_OVERFLOW) != 0u;
+  const bool overflowed = (*d.status & ST_HALT) != 0u;
   const unsigned long long mcount = *d.mcount;
   double r[K][3], u[K][3];
   int e0 = 0, ec[2] = {0, 0};  // the lane's pair slots: first, per bond

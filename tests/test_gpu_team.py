@@ -173,3 +173,28 @@ def test_layouts_of_two_contexts(blocks):
     for ctx in ctxs:
         ctx.close()
     oracle.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("name,scale", [("A", 0.05), ("B", 0.0204), ("B", 0.0206), ("E", 0.026)])
+def test_chained_runs_match_host_path(name, scale, precision):
+    """Small contexts' captured runs, launched without conditional nodes, take
+    the bits, lists and rebuild counts of host-driven steps: fewer bonds than
+    one block of the control kernel, just below and above one pass of its
+    cluster (4,096 bonds), and buckling filaments whose list outgrows its
+    storage inside a run."""
+    import simcore_b200 as sc
+    from simcore_b200 import workloads
+    cfg = workloads.make(name, scale=scale, seed=4, **(dict(n_seg=40) if name == "E" else {}))
+    a, b = (sc.Context(*cfg[:3], precision=precision) for _ in range(2))
+    for n in ((400,) if name == "E" else (40, 1, 23)):
+        a.step_graph(n)
+        b.step(n)
+        assert np.array_equal(a.sites(), b.sites())
+        assert all(np.array_equal(x, y) for x, y in zip(a.pairs(), b.pairs()))
+        ca, cb = a.counters(), b.counters()
+        assert (ca.i_step, ca.n_rebuilds) == (cb.i_step, cb.n_rebuilds)
+    assert name == "A" or ca.n_rebuilds > 1
+    assert name != "E" or ca.n_list_regrowths > 0
+    a.close()
+    b.close()
