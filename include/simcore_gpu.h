@@ -270,7 +270,9 @@ sc_status sc_update_positions(sc_ctx *ctx);
  * kernel and an integrator kernel.  Bit-identical to n x (sc_interact +
  * sc_update_positions). */
 sc_status sc_step(sc_ctx *ctx, int n);
-/* Same as sc_step, replaying a captured CUDA graph of n steps. */
+/* Same as sc_step without a host round trip per step: rebuilds are decided on
+ * the device, in a captured CUDA graph or, of small systems, a chain of
+ * launches. */
 sc_status sc_step_graph(sc_ctx *ctx, int n);
 /* Waits for the context's stream and reports any deferred device error. */
 sc_status sc_synchronize(sc_ctx *ctx);

@@ -159,7 +159,7 @@ class Simulation {
   // The step loop of Simulation::RunSimulation (src/simulation.cpp:37-62)
   // for n steps: ZeroForces (folded into Interact on the GPU), Interact,
   // Integrate.  With per_step_hook null the steps run back to back as one
-  // captured graph per call (sc_step_graph); otherwise host-driven, the hook
+  // run per call (sc_step_graph); otherwise host-driven, the hook
   // called after every step (where the reference runs Statistics and
   // WriteOutputs).
   template <class Hook>
