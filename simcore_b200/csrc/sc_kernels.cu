@@ -691,7 +691,8 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // The list and its slot indices date from the last rebuild, whose kernels
 // completed before the kernel just before this one waited (every kernel
 // waits before it lets the next one start): they are loaded before the
-// wait; the bond geometry, which that kernel may be writing, after it.
+// wait; the bond geometry, which that kernel may be writing, after it.  After a
+// chained step's control kernel, which may have rebuilt them, wait_first is set.
 template <int ND, int PREC, bool NPX, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
     k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first) {

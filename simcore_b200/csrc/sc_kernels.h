@@ -128,9 +128,10 @@ int launch_zero_dr(const DevState &d, cudaStream_t st);
 // npx (mixed only): nearly parallel pairs are evaluated in FP64 from the
 // sites, in place.  The kernel loads the pair list and slot indices before
 // it waits on the kernel launched just before it (programmatic dependent
-// launch): that kernel must not write them -- the last kernel of a rebuild
-// does not -- or the launch must be made without the overlap (PdlOff), or with
-// wait_first: the kernel waits before it loads anything.
+// launch): that kernel must not write them, or the launch must be made without
+// the overlap (PdlOff), or with wait_first: the kernel waits before it loads
+// anything.  (A host-driven rebuild, whose last kernel writes the slot indices,
+// ends with a synchronisation.)
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
                  int expected, cudaStream_t st, bool npx = false, int block = 256,
                  bool wait_first = false);
