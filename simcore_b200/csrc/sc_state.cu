@@ -149,7 +149,9 @@ sc_status sc_checkpoint(sc_ctx *c, void *buf, size_t cap, size_t *size) {
 // The index ranges of a checkpoint's pair lists, checked on the host before
 // anything is uploaded, so that no blob can send a later launch outside its
 // arrays: system r's live pairs join two of its bonds and write two of its
-// slots, and every entry of its bonds names one of its live pairs.
+// slots, every entry of its bonds names one of its live pairs, and a bond's
+// entries follow those of the filament's bond before it, as every rebuild lays
+// them out (a lane of the team integrator reads two bonds' slots as one run).
 sc_status check_pair_indices(sc_ctx *c, const std::vector<long long> &caps,
                              const std::vector<Region> &regions, const char *payload) {
   const int32_t *ix[RK_EENT + 1] = {};
@@ -174,6 +176,10 @@ sc_status check_pair_indices(sc_ctx *c, const std::vector<long long> &caps,
       const long long e0 = e_off[b], ec = e_cnt[b];
       if (ec < 0 || e0 < s0 || e0 + ec > s1)
         return fail(c, SC_ERR_INVALID_ARG, "checkpoint: bond %lld entries out of range", b);
+      if (b > R.b0 && c->bond_fil[b] == c->bond_fil[b - 1] &&
+          e0 != (long long)e_off[b - 1] + e_cnt[b - 1])
+        return fail(c, SC_ERR_INVALID_ARG,
+                    "checkpoint: bond %lld entries apart from its neighbour's", b);
       for (long long e = e0; e < e0 + ec; ++e)
         if (e_ent[e] < 0 || (e_ent[e] >> 1) < p0 || (e_ent[e] >> 1) >= p0 + n)
           return fail(c, SC_ERR_INVALID_ARG, "checkpoint: entry %lld out of range", e);
