@@ -75,10 +75,10 @@ sc::HostReport host_report(sc_ctx *c) {
 
 // Reads the status word, every system's displacement maximum and pair count.
 sc_status readback(sc_ctx *c) {
-  if (c->d.nrep > 0) {
+  if (c->loaded) {
     c->launches += sc::launch_report(c->d, host_report(c), 0, c->st);
     CK(cudaGetLastError());
-  } else {  // nothing loaded yet
+  } else {  // nothing loaded, or a failed load: not every array exists
     CK(cudaMemcpyAsync(&c->hb->status, c->d.status, sizeof(unsigned), cudaMemcpyDeviceToHost,
                        c->st));
   }
