@@ -427,11 +427,11 @@ sc_status layout_integrator(sc_ctx *c) {
     const int nn = off[f + 1] - off[f];
     if (nn > c->warp_sites) max_long = std::max(max_long, nn);
   }
-  c->C = c->block_sites > 0 ? c->block_sites
-                            : (max_long <= 128 ? 128 : max_long <= 256 ? 256 : 512);
-  if (max_long > c->C)
+  const int C = c->block_sites > 0 ? c->block_sites
+                                   : (max_long <= 128 ? 128 : max_long <= 256 ? 256 : 512);
+  if (max_long > C)
     return fail(c, SC_ERR_INVALID_ARG, "a %d-site filament does not fit %d-site blocks", max_long,
-                c->C);
+                C);
   const int team_max = c->warp_sites;
   auto sites = [&](int f) { return off[f + 1] - off[f]; };
   auto rep = [&](int f) { return c->fil_rep.empty() ? 0 : c->fil_rep[f]; };
@@ -483,7 +483,7 @@ sc_status layout_integrator(sc_ctx *c) {
   std::vector<int4> slots;
   for (const auto &ids : longs) {
     if (packed) {
-      for (const auto &bin : best_fit(ids, c->C, sites)) {
+      for (const auto &bin : best_fit(ids, C, sites)) {
         blk_site0.push_back(0);
         blk_f0.push_back((int)list.size());
         blk_nf.push_back((int)bin.size());
@@ -495,48 +495,64 @@ sc_status layout_integrator(sc_ctx *c) {
           slot += sites(bin[q]);
         }
         blk_ns.push_back(slot);
-        slots.resize(blk_f0.size() * (size_t)c->C, make_int4(off[bin[0]], bin[0], 0, 0));
+        slots.resize(blk_f0.size() * (size_t)C, make_int4(off[bin[0]], bin[0], 0, 0));
       }
       continue;
     }
     for (size_t i = 0; i < ids.size();) {
       const int f0 = ids[i], s0 = off[f0];
       int f = f0;
-      while (i < ids.size() && ids[i] == f && off[f + 1] - s0 <= c->C) ++i, ++f;
+      while (i < ids.size() && ids[i] == f && off[f + 1] - s0 <= C) ++i, ++f;
       blk_site0.push_back(s0);
       blk_f0.push_back(f0);
       blk_nf.push_back(f - f0);
       blk_ns.push_back(off[f] - s0);
     }
   }
+  // The new tables; when one cannot be made, the context keeps its old ones.
+  int *q_site0 = nullptr, *q_f0 = nullptr, *q_nf = nullptr, *q_ns = nullptr;
+  int2 *q_list = nullptr;
+  int4 *q_slot = nullptr, *q_lane = nullptr;
+  auto up = [&](auto **dst, const auto &v) -> sc_status {
+    using T = typename std::remove_reference<decltype(v)>::type::value_type;
+    CKS(dalloc(c, dst, v.size()));
+    if (!v.empty())
+      CK(cudaMemcpyAsync(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c->st));
+    return SC_OK;
+  };
+  auto all = [&]() -> sc_status {
+    CKS(up(&q_site0, blk_site0));
+    CKS(up(&q_f0, blk_f0));
+    CKS(up(&q_nf, blk_nf));
+    CKS(up(&q_ns, blk_ns));
+    CKS(up(&q_lane, lanes));
+    if (!slots.empty()) {
+      CKS(up(&q_list, list));
+      CKS(up(&q_slot, slots));
+    }
+    CK(cudaStreamSynchronize(c->st));
+    return SC_OK;
+  };
+  const sc_status made = all();
+  if (made != SC_OK) {
+    for (void *q : {(void *)q_site0, (void *)q_f0, (void *)q_nf, (void *)q_ns, (void *)q_list,
+                    (void *)q_slot, (void *)q_lane})
+      dfree(c, q);
+    return made;
+  }
   DevState &d = c->d;
   for (const void *q : {(const void *)d.blk_site0, (const void *)d.blk_f0, (const void *)d.blk_nf,
                         (const void *)d.blk_ns, (const void *)d.blk_list, (const void *)d.blk_slot,
                         (const void *)d.tm_lane})
     dfree(c, const_cast<void *>(q));
-  d.blk_site0 = d.blk_f0 = d.blk_nf = d.blk_ns = nullptr;  // (an upload below may fail)
-  d.blk_list = nullptr;
-  d.blk_slot = d.tm_lane = nullptr;
-  auto up = [&](auto **dst, const auto &v) -> sc_status {
-    using T = typename std::remove_reference<decltype(v)>::type::value_type;
-    T *q = nullptr;
-    *dst = nullptr;
-    CKS(dalloc(c, &q, v.size()));
-    if (!v.empty())
-      CK(cudaMemcpyAsync(q, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, c->st));
-    *dst = q;
-    return SC_OK;
-  };
-  CKS(up(&d.blk_site0, blk_site0));
-  CKS(up(&d.blk_f0, blk_f0));
-  CKS(up(&d.blk_nf, blk_nf));
-  CKS(up(&d.blk_ns, blk_ns));
-  CKS(up(&d.tm_lane, lanes));
-  if (!slots.empty()) {
-    CKS(up(&d.blk_list, list));
-    CKS(up(&d.blk_slot, slots));
-  }
-  CK(cudaStreamSynchronize(c->st));
+  d.blk_site0 = q_site0;
+  d.blk_f0 = q_f0;
+  d.blk_nf = q_nf;
+  d.blk_ns = q_ns;
+  d.blk_list = q_list;
+  d.blk_slot = q_slot;
+  d.tm_lane = q_lane;
+  c->C = C;
   d.blk_wide = packed && max_long - 1 > sc::kPcrMinRows ? 1 : 0;
   c->nblocks = (int)blk_f0.size();
   d.blk_maxf = 0;

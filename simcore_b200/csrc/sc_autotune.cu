@@ -15,10 +15,9 @@ sc_status sc_set_integrator_layout(sc_ctx *c, int warp_max_sites, int block_site
   c->warp_sites = warp_max_sites;
   c->block_sites = block_sites;
   sc_status st = layout_integrator(c);
-  if (st != SC_OK) {
+  if (st != SC_OK) {  // the tables are the old layout's
     c->warp_sites = ow;
     c->block_sites = ob;
-    layout_integrator(c);
   }
   return st;
 }
@@ -140,7 +139,7 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
   const int ow = c->warp_sites, ob = c->block_sites;
   const int interaction = c->desc.interaction_flag ? 1 : 0;
   float best = 1e30f;
-  std::pair<int, int> best_lay{ow, ob};
+  std::pair<int, int> best_lay{ow, ob}, laid{ow, ob};
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -150,6 +149,7 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
     c->block_sites = lay.second;
     st = layout_integrator(c);
     if (st != SC_OK) break;
+    laid = lay;
     for (int it = 0; it < 2; ++it)
       sc::launch_integrate(c->k, c->d, c->nblocks, c->C, 1 - it, c->rbuf, interaction, 0,
                            c->prec, c->fast, c->st, fuse);
@@ -197,7 +197,11 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
   CKS(copy_all(false));
   CK(cudaStreamSynchronize(c->st));
   dfree(c, save);
-  CKS(st);
+  if (st != SC_OK) {  // the last candidate that was laid out stays
+    c->warp_sites = laid.first;
+    c->block_sites = laid.second;
+    return st;
+  }
   c->warp_sites = best_lay.first;
   c->block_sites = best_lay.second;
   c->pair_block = best_pb;

@@ -1,22 +1,24 @@
 // A CUDA runtime without a GPU, preloaded by tests/test_failed_loading.py: device
 // memory is zeroed host memory, copies happen at once, kernels are counted and
-// not run.  The n-th allocation from now on can be made to fail.
+// not run.  The n-th allocation from now on, or all from then on, can be made to fail.
 #include <stdlib.h>
 #include <string.h>
 
 #define CUDA_OK 0
 #define CUDA_NO_MEMORY 2
-static long fail_in = -1, launches = 0, live = 0;
+static long fail_in = -1, fail_all = 0, launches = 0, live = 0;
 
 // Lets n allocations pass and fails the next one (n < 0: none).
-void fake_fail_after(long n) { fail_in = n; }
+void fake_fail_after(long n) { fail_in = n, fail_all = 0; }
+// The same, and fails every later one too.
+void fake_fail_from(long n) { fail_in = n, fail_all = 1; }
 long fake_launches(void) { return launches; }
 long fake_live(void) { return live; }
 
 static int take(void **p, size_t n) {
   *p = 0;
   if (fail_in == 0) {
-    fail_in = -1;
+    if (!fail_all) fail_in = -1;
     return CUDA_NO_MEMORY;
   }
   if (fail_in > 0) --fail_in;

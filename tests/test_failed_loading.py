@@ -1,5 +1,6 @@
-"""A context whose filaments could not be loaded, one allocation failing after
-another, on a CUDA runtime without a GPU (tests/native/fake_cudart.c)."""
+"""A context whose filaments could not be loaded or laid out anew, one allocation
+failing after another, on a CUDA runtime without a GPU
+(tests/native/fake_cudart.c)."""
 import os
 import subprocess
 import sys
@@ -15,7 +16,7 @@ sys.path.insert(0, %(root)r)
 import simcore_b200 as sc
 from simcore_b200 import workloads
 fake = ctypes.CDLL(%(fake)r)
-fake.fake_fail_after.argtypes = [ctypes.c_long]
+fake.fake_fail_after.argtypes = fake.fake_fail_from.argtypes = [ctypes.c_long]
 fake.fake_launches.restype = fake.fake_live.restype = ctypes.c_long
 cfg = workloads.make("C", scale=0.002, seed=1)
 
@@ -65,6 +66,25 @@ while True:
 assert n > 50
 """
 
+FAILED_LAYOUT = CHILD + r"""
+ctx = load(-1)
+assert not hasattr(ctx, "failed")
+live = fake.fake_live()
+n = 0
+while True:
+    fake.fake_fail_from(n)
+    rc = sc.lib.sc_set_integrator_layout(ctx.h, 0, 256)
+    fake.fake_fail_after(-1)
+    if rc == sc.SC_OK:
+        break
+    assert rc == 2, (n, rc)
+    assert fake.fake_live() == live, "the tables changed when allocation %%d failed" %% n
+    n += 1
+assert n > 3
+ctx.close()
+assert fake.fake_live() == 0
+"""
+
 
 def run_on_fake(tmp_path, code):
     """The code in a child process whose CUDA runtime is the fake."""
@@ -81,3 +101,9 @@ def test_synchronize_after_failed_loading_launches_nothing(tmp_path):
     """Whichever allocation of sc_add_filaments fails, sc_synchronize reads the
     status word and launches no kernel on arrays that do not exist."""
     run_on_fake(tmp_path, AFTER_FAILURE)
+
+
+def test_failed_layout_keeps_the_old_tables(tmp_path):
+    """When an allocation of a new integrator layout fails, and every one after
+    it, the context keeps the tables that its launches read."""
+    run_on_fake(tmp_path, FAILED_LAYOUT)
