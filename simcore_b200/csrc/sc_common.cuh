@@ -38,20 +38,6 @@ __device__ __forceinline__ void grid_dep_sync() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The same in two parts, for a kernel that runs beside the one before it: that
-// one's wait is enough for its own reads (it lets this one launch only after
-// it), it writes nothing that this one reads, and this one waits for it last,
-// so that whoever waits for this one has waited for both.  The fence keeps
-// this kernel's reads from being served from before it started (an L1 line
-// of an earlier kernel on the same SM): no wait of its own orders them.
-__device__ __forceinline__ void grid_dep_beside() {
-  __threadfence();
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void grid_dep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // Status bits set by kernels; the host maps them to sc_status codes.
 enum : unsigned {
   ST_NAN = 1u,            // non-finite position or force

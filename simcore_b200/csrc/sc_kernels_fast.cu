@@ -30,14 +30,13 @@ static void set_attr_fast(size_t smem) {
 // when the block has exactly MAXC.
 template <int ND, bool FUSE, int MAXC>
 static void launch_block_fast(const SysConst &k, const DevState &d, int nblocks, int C, size_t smem,
-                              int midstep, int rbuf, int interaction, int capture, int beside,
-                              cudaStream_t st) {
+                              int midstep, int rbuf, int interaction, int capture, cudaStream_t st) {
   if (C == MAXC)
     launch_pdl(k_integrate<ND, 1, true, MAXC, FUSE, true>, dim3(nblocks), dim3(C), smem, st, k, d,
-               midstep, rbuf, interaction, capture, beside);
+               midstep, rbuf, interaction, capture);
   else
     launch_pdl(k_integrate<ND, 1, true, MAXC, FUSE>, dim3(nblocks), dim3(C), smem, st, k, d,
-               midstep, rbuf, interaction, capture, beside);
+               midstep, rbuf, interaction, capture);
 }
 
 void prepare_integrate_fast(int C, size_t smem) {
@@ -60,6 +59,18 @@ template <int ND, bool FUSE>
 static int launch_fast(const SysConst &k, const DevState &d, int nblocks, int C, int midstep,
                        int rbuf, int interaction, int capture, cudaStream_t st) {
   int launched = 0;
+  if (nblocks > 0) {  // (before the team kernel: see launch_integrate)
+    const size_t smem = integrate_smem_bytes(C, d.blk_maxf);
+    if (C <= 128)
+      launch_block_fast<ND, FUSE, 128>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, st);
+    else if (C <= 192)
+      launch_block_fast<ND, FUSE, 192>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, st);
+    else if (C <= 256)
+      launch_block_fast<ND, FUSE, 256>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, st);
+    else
+      launch_block_fast<ND, FUSE, 512>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, st);
+    ++launched;
+  }
   if (d.n_tm > 0) {
     const int grid = (d.n_tm + kTeamWarps - 1) / kTeamWarps;
     if (d.tm_k == 1)
@@ -70,18 +81,7 @@ static int launch_fast(const SysConst &k, const DevState &d, int nblocks, int C,
                  team_smem_bytes(2), st, k, d, midstep, rbuf, interaction, capture);
     ++launched;
   }
-  if (nblocks == 0) return launched;
-  const int beside = launched;  // after the team kernel
-  const size_t smem = integrate_smem_bytes(C, d.blk_maxf);
-  if (C <= 128)
-    launch_block_fast<ND, FUSE, 128>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, beside, st);
-  else if (C <= 192)
-    launch_block_fast<ND, FUSE, 192>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, beside, st);
-  else if (C <= 256)
-    launch_block_fast<ND, FUSE, 256>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, beside, st);
-  else
-    launch_block_fast<ND, FUSE, 512>(k, d, nblocks, C, smem, midstep, rbuf, interaction, capture, beside, st);
-  return launched + 1;
+  return launched;
 }
 
 int launch_integrate_fast(const SysConst &k, const DevState &d, int nblocks, int C,

@@ -893,7 +893,7 @@ struct IntegrateBounds {
 template <int ND, int PREC, bool FAST, int MAXC, bool FUSE = false, bool FIXC = false>
 __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
     k_integrate(SysConst k, DevState d, int midstep, int rbuf, int interaction,
-                int capture, int beside) {
+                int capture) {
   extern __shared__ double smem[];
   const int C = FIXC ? MAXC : (int)blockDim.x;
   double *su = smem;            // site orientations    3C
@@ -936,10 +936,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   // Without a pair stage in between (fused pairs, or no interactions) the
   // kernel before this one may be the previous integrator step, whose
   // writes every load below reads: wait for it first.
-  // (beside: launched right after the team kernel of the same step, whose
-  // filaments are others; it has waited for what this one reads.)
-  if (beside) grid_dep_beside();
-  else if (FUSE || !interaction) grid_dep_sync();
+  if (FUSE || !interaction) grid_dep_sync();
   // A rebuild of this step whose list outgrew its segment stops the step
   // before its first store (uniform over the grid: nothing in this kernel
   // sets that bit), so the host can grow the list and redo the step.
@@ -1044,10 +1041,9 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   }
   // Everything above is the previous integrator step's or older; the pair
   // stage just before this kernel writes the bond slots read below.
-  if (!beside) grid_dep_sync();
+  grid_dep_sync();
   if (overflowed) {  // uniform over the grid
     cp_async_wait_all();  // no copy into this block's shared memory outlives it
-    if (beside) grid_dep_wait();
     return;
   }
   if (has_bond && interaction) {
@@ -1749,7 +1745,6 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
       atomicMax(&d.dr_max_bits[sfil[0].rep], (unsigned long long)__double_as_longlong(v));
     }
   }
-  if (beside) grid_dep_wait();
 #undef V
 }
 

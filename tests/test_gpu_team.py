@@ -198,3 +198,29 @@ def test_chained_runs_match_host_path(name, scale, precision):
     assert name != "E" or ca.n_list_regrowths > 0
     a.close()
     b.close()
+
+
+def test_mixed_lengths_repeated_runs_bitwise():
+    """A step of a mixed-length context is a block kernel and a team kernel on
+    one pair stage's slots, their launches overlapping: runs in every form take
+    the oracle's bits, each time."""
+    import simcore_b200 as sc
+    from checkers import Oracle
+    rng = np.random.default_rng(8)
+    n_seg = rng.integers(5, 90, size=240)
+    system, fils, sites = _lattice(3, n_seg, 100.0, seed=8)
+    oracle = Oracle(system, fils, sites)
+    want = []
+    for _ in range(4):
+        oracle.step(10)
+        want.append((oracle.sites(), oracle.bond_forces()))
+    assert len(oracle.pairs()) > 2000
+    for _ in range(6):
+        ctx = sc.Context(system, fils, sites, precision="fp64")
+        for i, (x, (f, t)) in enumerate(want):
+            (ctx.step_graph if i % 2 else ctx.step)(10)
+            assert np.array_equal(ctx.sites(), x)
+            gf, gt = ctx.bond_forces()
+            assert np.array_equal(gf, f) and np.array_equal(gt, t)
+        ctx.close()
+    oracle.close()
