@@ -274,6 +274,12 @@ sc_status sc_step(sc_ctx *ctx, int n);
  * the device, in a captured CUDA graph or, of small systems, a chain of
  * launches. */
 sc_status sc_step_graph(sc_ctx *ctx, int n);
+/* The form of sc_step_graph's runs: SC_RUN_AUTO (default) picks by the system's
+ * size, SC_RUN_GRAPH always replays the captured graph, SC_RUN_CHAIN always
+ * launches the steps one after another (systems without interactions have the
+ * graph alone).  Every form gives the same results. */
+typedef enum { SC_RUN_AUTO = 0, SC_RUN_GRAPH = 1, SC_RUN_CHAIN = 2 } sc_run_form;
+sc_status sc_set_run_form(sc_ctx *ctx, sc_run_form form);
 /* Waits for the context's stream and reports any deferred device error. */
 sc_status sc_synchronize(sc_ctx *ctx);
 

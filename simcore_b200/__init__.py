@@ -40,7 +40,8 @@ EXPORTED = ["sc_create", "sc_destroy", "sc_last_error", "sc_add_filaments",
             "sc_set_thermo", "sc_thermo_open", "sc_get_thermo", "sc_get_potential_energy",
             "sc_set_exact_near_parallel", "sc_set_near_parallel_threshold",
             "sc_set_fused_pairs", "sc_diffusion_init",
-            "sc_diffusion_sample", "sc_diffusion_results", "sc_insert_filaments_gpu"]
+            "sc_diffusion_sample", "sc_diffusion_results", "sc_insert_filaments_gpu",
+            "sc_set_run_form"]
 
 
 class ScError(RuntimeError):
@@ -188,6 +189,12 @@ class Context:
 
     def step_graph(self, n=1):
         self._check(lib.sc_step_graph(self.h, ctypes.c_int(n)))
+
+    def set_run_form(self, form="auto"):
+        """How step_graph runs: "auto" (by the system's size), "graph" (one
+        captured graph) or "chain" (launches one after another).  The results
+        are the same."""
+        self._check(lib.sc_set_run_form(self.h, {"auto": 0, "graph": 1, "chain": 2}[form]))
 
     def add_crosslinks(self, site_a, site_b, k_spring=10.0, k_spring_compress=-1.0,
                        rest_length=0.0):

@@ -121,6 +121,7 @@ struct sc_ctx {
   cudaGraphExec_t graph_exec = nullptr;
   int graph_rbuf = -1;             // geometry buffer parity the graph was built for
   int *h_loop = nullptr;           // pinned: BD steps to do, left undone
+  sc_run_form run_form = SC_RUN_AUTO;
 
   // optional per-launch timing of the step kernel (host-driven path)
   long long rebuild_kernels = 0;    // kernels in one rebuild sequence

@@ -134,6 +134,19 @@ static sc_status build_graph(sc_ctx *c) {
   return SC_OK;
 }
 
+// Whether a captured run is launched as a chain.
+static bool chained(const sc_ctx *c) {
+  if (!c->desc.interaction_flag || c->run_form == SC_RUN_GRAPH) return false;
+  return c->run_form == SC_RUN_CHAIN || (c->nb <= kChainBonds && c->rb.n_groups <= kChainGroups);
+}
+
+sc_status sc_set_run_form(sc_ctx *c, sc_run_form form) {
+  if (!c || (form != SC_RUN_AUTO && form != SC_RUN_GRAPH && form != SC_RUN_CHAIN))
+    return SC_ERR_INVALID_ARG;
+  c->run_form = form;
+  return SC_OK;
+}
+
 sc_status sc_step_graph(sc_ctx *c, int n) {
   if (!c || !c->loaded || n < 0) return SC_ERR_INVALID_ARG;
   CK(cudaSetDevice(c->desc.device));
@@ -159,8 +172,7 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
     // rebuild is redone host-side and the run resumes with that step.
     for (int attempt = 0; bd > 0; ++attempt) {
       if (attempt == 8) return fail(c, SC_ERR_LIST_OVERFLOW, "pair list kept overflowing inside captured runs");
-      const bool chain = c->desc.interaction_flag && c->nb <= kChainBonds &&
-                         c->rb.n_groups <= kChainGroups;
+      const bool chain = chained(c);
       if (!chain && (!c->graph_exec || c->graph_rbuf != c->rbuf)) CKS(build_graph(c));
       // The head reads the step count and the last node writes everything
       // the host looks at, both in pinned memory: no copies, one
