@@ -685,7 +685,10 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // list is the prefix of its segment; with several systems every slot checks
 // that it holds a current pair of its system.  A list that outgrew its segment
 // (the step stops, its rebuild is redone) has holes, whose entries nothing has
-// written: it is not evaluated.
+// written: it is not evaluated.  In a captured run (in_run) a stopped step
+// evaluates nothing: the forces stay the last step's, however many launches a
+// chain still holds.  (The halting bits are the rebuild's and the control
+// kernel's: as old as the list.)
 // NPX (mixed only): nearly parallel pairs are evaluated in FP64
 // (eval_near_parallel) by the thread that meets them.
 // The list and its slot indices date from the last rebuild, whose kernels
@@ -695,11 +698,13 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // chained step's control kernel, which may have rebuilt them, wait_first is set.
 template <int ND, int PREC, bool NPX, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
-    k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first) {
+    k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first, int in_run) {
   if (wait_first) grid_dep_sync();
+  const bool halted = in_run && (*d.status & ST_HALT) != 0u;
   if (d.nrep == 1) {
     const ReplicaConst &R = d.rep[0];
-    const int np = d.np_rep[0] <= R.pcap ? d.np_rep[0] : 0;
+    const int listed = d.np_rep[0];
+    const int np = halted | (listed > R.pcap) ? 0 : listed;  // (no branch: the loads are one trip)
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     PairIdx ix = {0, 0, 0, 0};
     if (p < np) ix = pair_idx(d, p);
@@ -721,7 +726,7 @@ __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.pcap_total;
        p += gridDim.x * blockDim.x) {
     int r;
-    if (pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap &&
+    if (!halted && pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap &&
         !pair_eval_one<ND, PREC, NPX>(k, d, d.rep[r], rbuf, p, pair_idx(d, p)))
       if (NPX) near_parallel_fp64<ND>(k, d, d.rep[r], p);
   }
@@ -755,6 +760,7 @@ __global__ void __launch_bounds__(128) k_mesh_lambda(DevState d) {
   grid_dep_sync();
   const int f = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (f >= d.nf) return;
+  if (*d.status & ST_HALT) return;  // the step stopped
   const int s0 = d.fil[f].site0, nbf = d.fil[f].n - 1, b0 = s0 - f;
   double true_length = 0.0;
   for (int q0 = 0; q0 < nbf; q0 += 32) {
@@ -1429,34 +1435,35 @@ int launch_zero_dr(const DevState &d, cudaStream_t st) {
 
 template <int BLOCK>
 static void launch_pairs_block(const SysConst &k, const DevState &d, int rbuf, int prec, int grid,
-                               cudaStream_t st, bool npx, int wait_first) {
+                               cudaStream_t st, bool npx, int wait_first, int in_run) {
   if (k.n_dim == 3) {
     if (prec == 0) launch_pdl(k_pair_eval<3, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first);
+                              wait_first, in_run);
     else if (!npx) launch_pdl(k_pair_eval<3, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                             wait_first);
+                              wait_first, in_run);
     else launch_pdl(k_pair_eval<3, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                    wait_first);
+                              wait_first, in_run);
   } else {
     if (prec == 0) launch_pdl(k_pair_eval<2, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first);
+                              wait_first, in_run);
     else if (!npx) launch_pdl(k_pair_eval<2, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                             wait_first);
+                              wait_first, in_run);
     else launch_pdl(k_pair_eval<2, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                    wait_first);
+                              wait_first, in_run);
   }
 }
 
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
-                 int expected, cudaStream_t st, bool npx, int block, bool wait_first) {
+                 int expected, cudaStream_t st, bool npx, int block, bool wait_first,
+                 bool in_run) {
   if (d.nrep > 1) expected = d.pcap_total;
   npx = npx && prec != 0;
   if (block == 128)
     launch_pairs_block<128>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 128), st, npx,
-                            wait_first);
+                            wait_first, in_run);
   else
     launch_pairs_block<256>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 256), st, npx,
-                            wait_first);
+                            wait_first, in_run);
   return 1;
 }
 

@@ -153,3 +153,27 @@ def test_default_form_at_its_limits(n_fil, side):
         ctxs[-1].step_graph(30)
     for other in ctxs[1:]:
         _same_run(ctxs[0], other)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_stopped_run_leaves_the_same_forces(precision):
+    """A run that an error stops leaves the forces of its last step, whichever
+    form it has: the launches that a chain still holds change nothing.  (A pair
+    out of range keeps its stored force, so an evaluation of the positions after
+    the last step would show.)"""
+    import simcore_b200 as sc
+    system, fils, sites = _workload("B", 0.05, seed=14)
+    got = []
+    for form in FORMS:
+        ctx = _ctx(system, fils, sites, precision)
+        ctx.set_run_form(form)
+        ctx.set_thermo(10**6)
+        ctx.step(2)
+        moved = ctx.sites()
+        moved[:11, 0] += 80.0
+        ctx.set_sites(moved)
+        with pytest.raises(sc.ScError):
+            ctx.step_graph(60)
+        got.append((ctx.sites(), ctx.pairs(), *ctx.bond_forces(), ctx.potential_energy()))
+    for x, y in zip(*got):
+        assert_same(x, y, "state after the stop")
