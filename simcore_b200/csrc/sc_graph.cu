@@ -15,6 +15,10 @@ using namespace scapi;
 // one counter per 32 cells; the suspensions of these sizes have up to 11,000.
 static const int kChainBonds = 12288;
 static const int kChainGroups = 32768;
+// BD steps queued at a time: what a run that stops early still launches for
+// nothing (about 2 us a launch), against a synchronisation and an empty queue
+// (about 15 us) per 9 ms or more of steps.
+static const int kChainPiece = 512;
 
 extern "C" {
 
@@ -170,17 +174,19 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
     // A rebuild whose list outgrows its segment stops the run at that BD
     // step, with nothing past the rebuild done; the list then grows, the
     // rebuild is redone host-side and the run resumes with that step.
-    for (int attempt = 0; bd > 0; ++attempt) {
+    // (A chain of more than kChainPiece steps is queued in pieces.)
+    for (int attempt = 0; bd > 0;) {
       if (attempt == 8) return fail(c, SC_ERR_LIST_OVERFLOW, "pair list kept overflowing inside captured runs");
       const bool chain = chained(c);
       if (!chain && (!c->graph_exec || c->graph_rbuf != c->rbuf)) CKS(build_graph(c));
       // The head reads the step count and the last node writes everything
       // the host looks at, both in pinned memory: no copies, one
       // synchronisation per launch.
-      *c->h_loop = bd;
+      const int queued = chain ? std::min(bd, kChainPiece) : bd;
+      *c->h_loop = queued;
       CK(cudaEventRecord(c->gev0, c->st));
       if (chain) {
-        enqueue_chain(c, bd);
+        enqueue_chain(c, queued);
         CK(cudaGetLastError());
       } else {
         CK(cudaGraphLaunch(c->graph_exec, c->st));
@@ -192,8 +198,9 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
       const unsigned st = c->hb->status;
       const long long nr0 = c->hb->rebuilds[0], nr1 = c->hb->rebuilds[1];
       const bool overflow = (st & sc::ST_LIST_OVERFLOW) != 0u;
-      // BD steps completed: all of them, or those before the stopped one.
-      const int done = overflow ? bd - *c->h_loop : bd;
+      // BD steps completed: all of them, or those before the stopped one.  (A run
+      // that an error ends counts as run to its end.)
+      const int done = overflow ? queued - *c->h_loop : st ? bd : queued;
       if (c->graph_fused && done > 0) c->slots_stale = true;
       c->i_step += 2 * (long long)done;
       if (c->desc.stoch_flag) c->mcount += done;
@@ -219,8 +226,9 @@ sc_status sc_step_graph(sc_ctx *c, int n) {
       bd -= done;
       if (!overflow) {
         CKS(check_status(c));  // status and maxima were read with the counters
-        break;
+        continue;
       }
+      ++attempt;
       if (st & ~sc::ST_LIST_OVERFLOW) {
         CKS(readback(c));  // reports the other error
         return fail(c, SC_ERR_LIST_OVERFLOW, "pair list overflow inside a captured run");

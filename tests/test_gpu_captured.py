@@ -177,3 +177,29 @@ def test_stopped_run_leaves_the_same_forces(precision):
         got.append((ctx.sites(), ctx.pairs(), *ctx.bond_forces(), ctx.potential_energy()))
     for x, y in zip(*got):
         assert_same(x, y, "state after the stop")
+
+
+def test_long_chain_is_queued_in_pieces():
+    """2,070 steps, 1,035 BD steps, are three pieces of a chain (512 each): the
+    graph's bits.  A run that stops in its first piece launches no more of it:
+    the 4,000 steps of a run with an unphysical displacement would be 10,002
+    launches, a piece is 512 times five (control, two pair and two integrator
+    kernels) and three."""
+    import simcore_b200 as sc
+    system, fils, sites = _workload("B", 0.02, seed=14)
+    runs = []
+    for form in FORMS:
+        ctx = _ctx(system, fils, sites)
+        ctx.set_run_form(form)
+        ctx.step_graph(2070)
+        runs.append(ctx)
+    _same_run(*runs)
+    ctx = runs[1]
+    moved = ctx.sites()
+    moved[:11, 0] += 80.0
+    ctx.set_sites(moved)
+    before = ctx.counters().kernel_launches
+    with pytest.raises(sc.ScError) as e:
+        ctx.step_graph(4000)
+    assert e.value.code == 7
+    assert ctx.counters().kernel_launches - before <= 512 * 5 + 3
