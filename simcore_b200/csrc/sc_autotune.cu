@@ -22,10 +22,17 @@ sc_status sc_set_integrator_layout(sc_ctx *c, int warp_max_sites, int block_site
   return st;
 }
 
+// Version of the cached choices: raised when the integrator kernels change, so
+// that a choice made for others is not taken over.
+static const char kCacheVersion[] = "v4";
+
 // Autotuner.  Candidate integrator layouts (team kernel or not, block size)
 // and pair-kernel block sizes (128 or 256 threads) are timed on the
 // context's own state: the arrays they write are saved first and restored
-// afterwards, so the simulation is unchanged.  The fastest choices are
+// afterwards, so the simulation is unchanged.  An integrator is timed behind the
+// pair stage, as a step runs it: it does part of its work before it waits for
+// the kernel before it, on sites that an integrator launched just before it
+// would still be writing.  The fastest choices are
 // applied and, with a cache file, recorded per shape (device, precision,
 // filament count and site range) so later contexts skip the timing.
 sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
@@ -42,8 +49,8 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
   }
   char key[512];
   const bool fuse = fused_pairs(c);
-  std::snprintf(key, sizeof(key), "v3|%s|sm%d|nd%d|prec%d|fast%d|fuse%d|nf%d|ns%d|n%d-%d",
-                prop.name, prop.multiProcessorCount, c->nd, c->prec,
+  std::snprintf(key, sizeof(key), "%s|%s|sm%d|nd%d|prec%d|fast%d|fuse%d|nf%d|ns%d|n%d-%d",
+                kCacheVersion, prop.name, prop.multiProcessorCount, c->nd, c->prec,
                 (c->prec == 1 && c->fast) ? 1 : 0, fuse ? 1 : 0, c->nf, c->ns, min_n, max_n);
   auto finish = [&](int w, int b) -> sc_status {
     if (warp_sites_out) *warp_sites_out = w;
@@ -150,13 +157,15 @@ sc_status sc_autotune(sc_ctx *c, const char *cache_path, int *warp_sites_out,
     st = layout_integrator(c);
     if (st != SC_OK) break;
     laid = lay;
-    for (int it = 0; it < 2; ++it)
-      sc::launch_integrate(c->k, c->d, c->nblocks, c->C, 1 - it, c->rbuf, interaction, 0,
+    auto step = [&](int midstep) {
+      if (interaction && !fuse)
+        sc::launch_pairs(c->k, c->d, c->rbuf, c->prec, (int)c->np, c->st, c->npx, c->pair_block);
+      sc::launch_integrate(c->k, c->d, c->nblocks, c->C, midstep, c->rbuf, interaction, 0,
                            c->prec, c->fast, c->st, fuse);
+    };
+    for (int it = 0; it < 2; ++it) step(1 - it);
     cudaEventRecord(e0, c->st);
-    for (int it = 0; it < 8; ++it)
-      sc::launch_integrate(c->k, c->d, c->nblocks, c->C, 1 - (it & 1), c->rbuf, interaction, 0,
-                           c->prec, c->fast, c->st, fuse);
+    for (int it = 0; it < 8; ++it) step(1 - (it & 1));
     cudaEventRecord(e1, c->st);
     if (cudaEventSynchronize(e1) != cudaSuccess) {
       st = fail(c, SC_ERR_CUDA, "autotune: %s", cudaGetErrorString(cudaGetLastError()));

@@ -224,3 +224,28 @@ def test_mixed_lengths_repeated_runs_bitwise():
             assert np.array_equal(gf, f) and np.array_equal(gt, t)
         ctx.close()
     oracle.close()
+
+
+def test_autotune_cache_of_other_kernels_is_not_read(tmp_path):
+    """A cached choice made for earlier integrator kernels (the third version
+    of the cache) is left alone, and the shape is timed again."""
+    import simcore_b200 as sc
+    system, fils, sites = _lattice(3, np.array([10] * 200), 60.0, seed=2)
+    cache = tmp_path / "tune.txt"
+    a = sc.Context(system, fils, sites, precision="fp64")
+    lay = a.autotune(str(cache))
+    line = cache.read_text()
+    key = line.split("|", 1)[1]
+    other = "0 512 1.00 128"
+    cache.write_text("v3|" + key.split("\t")[0] + "\t" + other + "\n")
+    b = sc.Context(system, fils, sites, precision="fp64")
+    b.autotune(str(cache))
+    lines = cache.read_text().splitlines()
+    assert len(lines) == 2 and lines[1].split("\t")[0] == line.split("\t")[0]
+    # Each context goes on as an untuned one.
+    c = sc.Context(system, fils, sites, precision="fp64")
+    for ctx in (a, b, c):
+        ctx.step(3)
+        ctx.step_graph(4)
+    assert np.array_equal(a.sites(), c.sites()) and np.array_equal(b.sites(), c.sites())
+    assert lay[0] in (0, 32)
