@@ -380,30 +380,66 @@ sc_status maybe_rebuild(sc_ctx *c) {
   return rebuild(c);
 }
 
-// Whole filaments `ids` into bins of `cap` by their sizes, best fit in order
-// of decreasing size (equal sizes in filament order): the bins' filaments.
+// Filaments in bins, bin after bin: bin i holds ids[first[i]] .. ids[first[i + 1] - 1].
+struct Bins {
+  std::vector<int> ids, first{0};
+  int count() const { return (int)first.size() - 1; }
+};
+
+// Whole filaments `ids` into bins of `cap` (at most 512) by their sizes, best
+// fit in order of decreasing size (equal sizes in filament order, and of several
+// bins with as much room the one used last).  Equal filaments fill the bins in
+// order.  The bins' rooms are lists through the bins, found by a bit per room:
+// about 20 ns a filament of 4,000 mixed ones (3 equal ones), where a vector per
+// bin and per room took 100 to 190 (40 to 130).
 template <class Size>
-static std::vector<std::vector<int>> best_fit(std::vector<int> ids, int cap, Size &&size) {
-  std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return size(a) > size(b); });
-  std::vector<std::vector<int>> bins;
-  std::vector<std::vector<int>> room(cap + 1);  // bins by what they still hold
-  for (int f : ids) {
-    const int need = size(f);
-    int left = need;
-    while (left <= cap && room[left].empty()) ++left;
-    int bin;
-    if (left <= cap) {
-      bin = room[left].back();
-      room[left].pop_back();
-    } else {
-      left = cap;
-      bin = (int)bins.size();
-      bins.emplace_back();
-    }
-    bins[bin].push_back(f);
-    room[left - need].push_back(bin);
+static Bins best_fit(const std::vector<int> &ids, int cap, Size &&size) {
+  Bins out;
+  const int n = (int)ids.size();
+  if (n == 0) return out;
+  std::vector<int> begin(cap + 2, 0);  // of the sizes, largest first
+  for (int f : ids) ++begin[cap - size(f) + 1];
+  if (begin[cap - size(ids[0]) + 1] == n) {
+    const int per = cap / size(ids[0]);
+    out.ids = ids;
+    for (int i = per; i < n; i += per) out.first.push_back(i);
+    out.first.push_back(n);
+    return out;
   }
-  return bins;
+  for (int q = 0; q <= cap; ++q) begin[q + 1] += begin[q];
+  std::vector<int> order(n), bin_of(n), next, fill;  // per filament; per bin
+  for (int f : ids) order[begin[cap - size(f)]++] = f;
+  std::vector<int> room(cap + 1, -1);  // the bin used last of those with this much room
+  unsigned long long open[9] = {};     // whether there is one
+  auto put = [&](int left, int bin) {
+    next[bin] = room[left];
+    room[left] = bin;
+    open[left >> 6] |= 1ull << (left & 63);
+  };
+  for (int i = 0; i < n; ++i) {
+    const int need = size(order[i]);
+    int w = need >> 6;
+    unsigned long long bits = open[w] & (~0ull << (need & 63));
+    while (!bits && ++w < 9) bits = open[w];
+    int left = cap, bin = (int)next.size();
+    if (bits) {
+      left = w << 6 | __builtin_ctzll(bits);
+      bin = room[left];
+      room[left] = next[bin];
+      if (room[left] < 0) open[w] &= ~(1ull << (left & 63));
+    } else {
+      next.push_back(-1);
+      fill.push_back(0);
+    }
+    bin_of[i] = bin;
+    ++fill[bin];
+    put(left - need, bin);
+  }
+  for (int v : fill) out.first.push_back(out.first.back() + v);
+  out.ids.resize(n);
+  std::vector<int> at(out.first.begin(), out.first.end() - 1);
+  for (int i = 0; i < n; ++i) out.ids[at[bin_of[i]]++] = order[i];
+  return out;
 }
 
 // Integrator work units: filaments of at most warp_sites sites each go to the
@@ -456,25 +492,39 @@ sc_status layout_integrator(sc_ctx *c) {
   // an SM instead of 20, so two pay where they save more than half the warps
   // (the margin covers 20,000 filaments of 5 to 32 sites, 1.9 times fewer:
   // 35 us with one, 50 with two) and one lane a site fills the chip at all.
-  std::vector<std::vector<int>> teams[3];
-  for (int k = 1; k <= 2; ++k)
-    for (const auto &ids : shorts)
-      for (auto &bin : best_fit(ids, 32, [&](int f) { return (sites(f) + k - 1) / k; }))
-        teams[k].push_back(std::move(bin));
-  const int K = teams[1].size() > 148 * 20 && 4 * teams[1].size() >= 9 * teams[2].size() ? 2 : 1;
+  auto pack_teams = [&](int k, std::vector<Bins> &teams) {
+    long long warps = 0;
+    for (const auto &ids : shorts) {
+      teams.push_back(best_fit(ids, 32, [&](int f) { return (sites(f) + k - 1) / k; }));
+      warps += teams.back().count();
+    }
+    return warps;
+  };
+  int K = 1;
+  std::vector<Bins> teams, teams2;
+  const long long warps = pack_teams(1, teams);
+  if (warps > 148 * 20 && 4 * warps >= 9 * pack_teams(2, teams2)) {
+    K = 2;
+    teams.swap(teams2);
+  }
   const bool uni = equal && one_system && sites(0) <= team_max;
   std::vector<int4> lanes;
-  if (!uni)
-    for (const auto &bin : teams[K]) {
-      const size_t base = lanes.size();
-      for (size_t q = 0; q < bin.size(); ++q)
-        for (int j = 0; j < sites(bin[q]); j += K)
-          lanes.push_back(make_int4(off[bin[q]] + j, bin[q], j | sites(bin[q]) << 16,
-                                    (int)q | (int)bin.size() << 8));
-      // Idle lanes name the warp's first site, of a filament without sites.
-      while (lanes.size() < base + 32)
-        lanes.push_back(make_int4(off[bin[0]], bin[0], 0, (int)bin.size() << 8));
-    }
+  if (!uni) {
+    lanes.reserve(32 * (size_t)std::accumulate(teams.begin(), teams.end(), 0ll,
+                                               [](long long x, const Bins &b) { return x + b.count(); }));
+    for (const Bins &bins : teams)
+      for (int i = 0; i < bins.count(); ++i) {
+        const int *bin = &bins.ids[bins.first[i]], nfw = bins.first[i + 1] - bins.first[i];
+        const size_t base = lanes.size();
+        for (int q = 0; q < nfw; ++q) {
+          const int o = off[bin[q]], nn = sites(bin[q]);
+          for (int j = 0; j < nn; j += K)
+            lanes.push_back(make_int4(o + j, bin[q], j | nn << 16, q | nfw << 8));
+        }
+        // Idle lanes name the warp's first site, of a filament without sites.
+        lanes.resize(base + 32, make_int4(off[bin[0]], bin[0], 0, nfw << 8));
+      }
+  }
   // Blocks: of packed ones, their filaments with their first slots, and every
   // slot's site; of runs, their first site and filament.
   const bool packed = !equal && (c->prec == 0 || c->warp_sites >= 32);
@@ -483,16 +533,21 @@ sc_status layout_integrator(sc_ctx *c) {
   std::vector<int4> slots;
   for (const auto &ids : longs) {
     if (packed) {
-      for (const auto &bin : best_fit(ids, C, sites)) {
+      const Bins bins = best_fit(ids, C, sites);
+      list.reserve(list.size() + ids.size());
+      slots.reserve(slots.size() + (size_t)bins.count() * C);
+      for (int i = 0; i < bins.count(); ++i) {
+        const int *bin = &bins.ids[bins.first[i]], nfb = bins.first[i + 1] - bins.first[i];
         blk_site0.push_back(0);
         blk_f0.push_back((int)list.size());
-        blk_nf.push_back((int)bin.size());
+        blk_nf.push_back(nfb);
         int slot = 0;
-        for (size_t q = 0; q < bin.size(); ++q) {
+        for (int q = 0; q < nfb; ++q) {
+          const int o = off[bin[q]], nn = sites(bin[q]);
           list.push_back(make_int2(bin[q], slot));
-          for (int j = 0; j < sites(bin[q]); ++j)
-            slots.push_back(make_int4(off[bin[q]] + j, bin[q], j | sites(bin[q]) << 16, (int)q));
-          slot += sites(bin[q]);
+          for (int j = 0; j < nn; ++j)
+            slots.push_back(make_int4(o + j, bin[q], j | nn << 16, q));
+          slot += nn;
         }
         blk_ns.push_back(slot);
         slots.resize(blk_f0.size() * (size_t)C, make_int4(off[bin[0]], bin[0], 0, 0));

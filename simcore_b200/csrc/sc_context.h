@@ -19,6 +19,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <numeric>
 #include <string>
 #include <type_traits>
 #include <vector>
