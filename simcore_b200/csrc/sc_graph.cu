@@ -38,7 +38,7 @@ static int bd_step(sc_ctx *c, bool fuse, bool chain) {
       std::optional<sc::PdlOff> alone;
       if (half == 0 && !chain) alone.emplace();
       n += sc::launch_pairs(c->k, c->d, rb, c->prec, (int)(c->np + c->np / 8), c->st, c->npx,
-                            c->pair_block, half == 0 && chain, true);
+                            c->pair_block, half == 0 && chain, chain);
     }
     if (interaction && c->k.thermo) n += sc::launch_thermo(c->k, c->d, c->prec, c->st);
     if (half == 0 && (!interaction || fuse)) {

@@ -685,10 +685,11 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // list is the prefix of its segment; with several systems every slot checks
 // that it holds a current pair of its system.  A list that outgrew its segment
 // (the step stops, its rebuild is redone) has holes, whose entries nothing has
-// written: it is not evaluated.  In a captured run (in_run) a stopped step
-// evaluates nothing: the forces stay the last step's, however many launches a
+// written: it is not evaluated.  In a chained run (chained) a stopped step
+// evaluates nothing: the forces stay the last step's, however many launches the
 // chain still holds.  (The halting bits are the rebuild's and the control
-// kernel's: as old as the list.)
+// kernel's: as old as the list.  A graph holds none past the step that stops it,
+// and the load costs several systems' larger lists 0.4 us a launch.)
 // NPX (mixed only): nearly parallel pairs are evaluated in FP64
 // (eval_near_parallel) by the thread that meets them.
 // The list and its slot indices date from the last rebuild, whose kernels
@@ -698,9 +699,9 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // chained step's control kernel, which may have rebuilt them, wait_first is set.
 template <int ND, int PREC, bool NPX, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
-    k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first, int in_run) {
+    k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first, int chained) {
   if (wait_first) grid_dep_sync();
-  const bool halted = in_run && (*d.status & ST_HALT) != 0u;
+  const bool halted = chained && (*d.status & ST_HALT) != 0u;
   if (d.nrep == 1) {
     const ReplicaConst &R = d.rep[0];
     const int listed = d.np_rep[0];
@@ -726,7 +727,7 @@ __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.pcap_total;
        p += gridDim.x * blockDim.x) {
     int r;
-    if (!halted && pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap &&
+    if (pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap && !halted &&
         !pair_eval_one<ND, PREC, NPX>(k, d, d.rep[r], rbuf, p, pair_idx(d, p)))
       if (NPX) near_parallel_fp64<ND>(k, d, d.rep[r], p);
   }
@@ -1435,35 +1436,35 @@ int launch_zero_dr(const DevState &d, cudaStream_t st) {
 
 template <int BLOCK>
 static void launch_pairs_block(const SysConst &k, const DevState &d, int rbuf, int prec, int grid,
-                               cudaStream_t st, bool npx, int wait_first, int in_run) {
+                               cudaStream_t st, bool npx, int wait_first, int chained) {
   if (k.n_dim == 3) {
     if (prec == 0) launch_pdl(k_pair_eval<3, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
     else if (!npx) launch_pdl(k_pair_eval<3, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
     else launch_pdl(k_pair_eval<3, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
   } else {
     if (prec == 0) launch_pdl(k_pair_eval<2, 0, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
     else if (!npx) launch_pdl(k_pair_eval<2, 1, false, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
     else launch_pdl(k_pair_eval<2, 1, true, BLOCK>, dim3(grid), dim3(BLOCK), 0, st, k, d, rbuf,
-                              wait_first, in_run);
+                              wait_first, chained);
   }
 }
 
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
                  int expected, cudaStream_t st, bool npx, int block, bool wait_first,
-                 bool in_run) {
+                 bool chained) {
   if (d.nrep > 1) expected = d.pcap_total;
   npx = npx && prec != 0;
   if (block == 128)
     launch_pairs_block<128>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 128), st, npx,
-                            wait_first, in_run);
+                            wait_first, chained);
   else
     launch_pairs_block<256>(k, d, rbuf, prec, cdiv(expected > 0 ? expected : 1, 256), st, npx,
-                            wait_first, in_run);
+                            wait_first, chained);
   return 1;
 }
 

@@ -131,11 +131,11 @@ int launch_zero_dr(const DevState &d, cudaStream_t st);
 // launch): that kernel must not write them, or the launch must be made without
 // the overlap (PdlOff), or with wait_first: the kernel waits before it loads
 // anything.  (A host-driven rebuild, whose last kernel writes the slot indices,
-// ends with a synchronisation.)  in_run: a step of a captured run, which does
+// ends with a synchronisation.)  chained: a step of a chained run, which does
 // nothing once the run has stopped.
 int launch_pairs(const SysConst &k, const DevState &d, int rbuf, int prec,
                  int expected, cudaStream_t st, bool npx = false, int block = 256,
-                 bool wait_first = false, bool in_run = false);
+                 bool wait_first = false, bool chained = false);
 // Crosslink tethers of an even step into the per-anchor contributions.
 int launch_tether(const SysConst &k, const DevState &d, cudaStream_t st);
 // Thermo: one step's pair virial per system, the pressure record every
