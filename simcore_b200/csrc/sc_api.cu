@@ -531,11 +531,19 @@ sc_status layout_integrator(sc_ctx *c) {
   std::vector<int> blk_site0, blk_f0, blk_nf, blk_ns;
   std::vector<int2> list;
   std::vector<int4> slots;
-  for (const auto &ids : longs) {
+  std::vector<Bins> blocks;  // packed, one per system
+  if (packed) {
+    long long most = 0;
+    for (const auto &ids : longs) {
+      blocks.push_back(best_fit(ids, C, sites));
+      most += blocks.back().count();
+    }
+    slots.reserve((size_t)most * C);
+  }
+  for (size_t sys = 0; sys < longs.size(); ++sys) {
+    const std::vector<int> &ids = longs[sys];
     if (packed) {
-      const Bins bins = best_fit(ids, C, sites);
-      list.reserve(list.size() + ids.size());
-      slots.reserve(slots.size() + (size_t)bins.count() * C);
+      const Bins &bins = blocks[sys];
       for (int i = 0; i < bins.count(); ++i) {
         const int *bin = &bins.ids[bins.first[i]], nfb = bins.first[i + 1] - bins.first[i];
         blk_site0.push_back(0);
