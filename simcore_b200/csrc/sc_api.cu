@@ -449,12 +449,11 @@ static Bins best_fit(const std::vector<int> &ids, int cap, Size &&size) {
 // others are packed by size, since runs of consecutive ones leave a third of a
 // 256-site block empty (20,000 filaments of 5 to 200 bonds: 233 us a launch for
 // those above 32 sites in runs, 173 packed; FP64 57.5 and 37.8 for 4,000 of 5 to
-// 100).  A filament's
-// results do not depend on its unit, but the fast integrator's blocks of more
-// than 128 sites draw and project the noise in FP64 when one of their
-// filaments has more than kPcrMinRows bonds: packed, all of them do (blk_wide)
-// if any filament has, and with short filaments in the blocks (warp_sites
-// below 32) the runs stay as they are.
+// 100).  A filament's results do not depend on its unit, but the fast
+// integrator's blocks of more than 128 sites draw and project the noise in FP64
+// when one of their filaments has more than kPcrMinRows bonds: packed, all of a
+// system's blocks do if any of its filaments has, and with short filaments in
+// the blocks (warp_sites below 32) the runs stay as they are.
 sc_status layout_integrator(sc_ctx *c) {
   const std::vector<int> &off = c->site_off;
   const int n = c->nf;
@@ -544,6 +543,8 @@ sc_status layout_integrator(sc_ctx *c) {
     const std::vector<int> &ids = longs[sys];
     if (packed) {
       const Bins &bins = blocks[sys];
+      int rows = 0;  // of the system's longest filament
+      for (int f : ids) rows = std::max(rows, sites(f) - 1);
       for (int i = 0; i < bins.count(); ++i) {
         const int *bin = &bins.ids[bins.first[i]], nfb = bins.first[i + 1] - bins.first[i];
         blk_site0.push_back(0);
@@ -557,7 +558,7 @@ sc_status layout_integrator(sc_ctx *c) {
             slots.push_back(make_int4(o + j, bin[q], j | nn << 16, q));
           slot += nn;
         }
-        blk_ns.push_back(slot);
+        blk_ns.push_back(slot | (rows > sc::kPcrMinRows ? sc::kBlockWide : 0));
         slots.resize(blk_f0.size() * (size_t)C, make_int4(off[bin[0]], bin[0], 0, 0));
       }
       continue;
@@ -616,7 +617,6 @@ sc_status layout_integrator(sc_ctx *c) {
   d.blk_slot = q_slot;
   d.tm_lane = q_lane;
   c->C = C;
-  d.blk_wide = packed && max_long - 1 > sc::kPcrMinRows ? 1 : 0;
   c->nblocks = (int)blk_f0.size();
   d.blk_maxf = 0;
   for (int v : blk_nf) d.blk_maxf = std::max(d.blk_maxf, v);

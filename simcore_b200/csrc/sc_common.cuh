@@ -111,6 +111,8 @@ struct ReplicaConst {
 // fast 256- and 512-site integrator blocks solve by pcr_block instead of
 // Thomas lanes.
 constexpr int kPcrMinRows = 32;
+// In a packed block's site count: its system has a filament of more rows.
+constexpr int kBlockWide = 1 << 16;
 
 // Per-filament constants of the integrator.  The reciprocals are the
 // reference's own quotients (1.0 / friction_par_, 2.0 / friction_perp_, ...,
@@ -146,14 +148,13 @@ struct DevState {
   const int *blk_site0;    // per block: first site
   const int *blk_f0;       // per block: first filament
   const int *blk_nf;       // per block: filament count
-  const int *blk_ns;       // per block: site count
+  const int *blk_ns;       // per block: site count (| kBlockWide)
   int blk_maxf;            // most filaments in one block (shared-memory size)
   // Packed blocks (null: runs of consecutive filaments): per block, from
   // blk_f0, its filaments with their first slots; per slot its site, its
   // filament, its index | filament sites << 16, its filament in the block.
   const int2 *blk_list;
   const int4 *blk_slot;
-  int blk_wide;            // a packed block's filament has more than kPcrMinRows bonds
   // Equal filaments of blk_uni_n sites, blk_uni_fpb to a block, every block
   // but the last full, sites numbered filament by filament from 0: blocks
   // and sites then find their filaments by arithmetic (0: read the tables).

@@ -944,6 +944,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   const unsigned long long mcount = *d.mcount;
   const int un = d.blk_uni_n;
   int s0, count, f0, nfb;
+  bool wide = false;
   if (un > 0) {  // equal filaments: the block's range without a table load
     f0 = blk * d.blk_uni_fpb;
     nfb = min(d.blk_uni_fpb, d.nf - f0);
@@ -952,6 +953,8 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   } else {
     s0 = d.blk_site0[blk];
     count = d.blk_ns[blk];
+    wide = count >= kBlockWide;
+    count &= kBlockWide - 1;
     f0 = d.blk_f0[blk];
     nfb = d.blk_nf[blk];
   }
@@ -1070,7 +1073,7 @@ __global__ void __launch_bounds__(MAXC, IntegrateBounds<MAXC, FAST>::min_blocks)
   int max_rows = 0;
   if (FAST && MAXC > 128)
     for (int q = 0; q < nfb; ++q) max_rows = max(max_rows, sfil[q].n - 1);
-  const bool pcr = FAST && MAXC > 128 && (d.blk_wide || max_rows > kPcrMinRows);
+  const bool pcr = FAST && MAXC > 128 && (wide || max_rows > kPcrMinRows);
   // First slot of the block's filament q.
   auto slot_of = [&](int q) { return sfil[q].site0 - s0; };
   // Sequential solves of the fast step: from both ends on lanes 2q, 2q+1 (of

@@ -249,3 +249,31 @@ def test_autotune_cache_of_other_kernels_is_not_read(tmp_path):
         ctx.step_graph(4)
     assert np.array_equal(a.sites(), c.sites()) and np.array_equal(b.sites(), c.sites())
     assert lay[0] in (0, 32)
+
+
+def test_noise_precision_follows_the_system():
+    """The fast blocks of a system whose longest filaments have 33 sites draw
+    the noise in FP32, whatever the other systems of the context hold: each of
+    two systems gives the bits it gives alone with the same block size."""
+    import simcore_b200 as sc
+    parts = [_lattice(2, np.array([32, 32, 9, 32, 20, 32, 32]), 330.0, seed=3),
+             _lattice(2, np.array([100, 7, 32, 70, 32]), 330.0, seed=4)]
+    fils = parts[0][1] + parts[1][1]
+    sites = np.concatenate([parts[0][2], parts[1][2]])
+    replicas = [dict(system_radius=p[0]["system_radius"], seed=p[0]["seed"],
+                     n_filaments=len(p[1])) for p in parts]
+    both = sc.Context(parts[0][0], fils, sites, precision="mixed", replicas=replicas)
+    both.set_integrator_layout(32, 256)
+    both.step(4)
+    alone = []
+    for system, f, x in parts:
+        ctx = sc.Context(system, f, x, precision="mixed")
+        ctx.set_integrator_layout(32, 256)
+        ctx.step(4)
+        alone.append(ctx.sites())
+        ctx.close()
+    n = len(alone[0])
+    got = both.sites()
+    assert np.array_equal(got[n:], alone[1])
+    assert np.array_equal(got[:n], alone[0])
+    both.close()
