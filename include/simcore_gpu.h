@@ -381,7 +381,7 @@ sc_status sc_get_graph_time(sc_ctx *ctx, double *ms);
 #define SC_NOALLOC_MAX_BONDS 8192
 #define SC_NOALLOC_MAX_CELLS 131072
 #define SC_NOALLOC_MAX_PAIRS 32768
-#define SC_NOALLOC_SCRATCH_BYTES 8882432 /* 8.5 MiB per GPU */
+#define SC_NOALLOC_SCRATCH_BYTES 7899392 /* 7.5 MiB per GPU */
 sc_status sc_pair_forces_noalloc(const sc_system_desc *desc,
                                  const sc_filament_params *species, int n_filaments,
                                  const int32_t *d_site_offsets, const double *d_site_xyz,

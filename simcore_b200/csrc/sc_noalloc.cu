@@ -11,7 +11,7 @@
 // stream, so it is called outside stream capture.
 //
 // The scratch is one file-scope __device__ array (g_noalloc_scratch below,
-// SC_NOALLOC_SCRATCH_BYTES = 8.5 MiB).  Every GPU that loads the library
+// SC_NOALLOC_SCRATCH_BYTES = 7.5 MiB).  Every GPU that loads the library
 // holds it until the process exits.  All calls on a device share it and it
 // keeps the last call's contents, so every call clears what must start at
 // zero; calls whose GPU work overlaps (several host threads, or several
@@ -45,9 +45,9 @@ constexpr int kMaxPairs = SC_NOALLOC_MAX_PAIRS;
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct Layout {
-  size_t r, key, cell_count, cell_start, sorted, pair_count, pair_off, deg, deg_off, e_off,
-      e_cnt, scan_tmp, bond_fil, ub, g64, pa, pb, pos1, pos2, pf, cf, e_ent, bF, bT, status,
-      counters, rep, sys, total;
+  size_t key, cell_count, cell_start, sorted, pair_count, pair_off, deg, deg_off, e_off, e_cnt,
+      scan_tmp, bond_fil, g64, pa, pb, pos1, pos2, pf, cf, e_ent, status, counters, rep, sys,
+      total;
 };
 
 constexpr int kScanTmp = (kMaxCells > kMaxBonds ? kMaxCells : kMaxBonds) / 2048 + 2;
@@ -55,7 +55,6 @@ constexpr int kScanTmp = (kMaxCells > kMaxBonds ? kMaxCells : kMaxBonds) / 2048 
 constexpr Layout make_layout() {
   Layout L{};
   size_t o = 0;
-  L.r = o;          o = align256(o + sizeof(double) * 3 * kMaxSites);
   L.key = o;        o = align256(o + sizeof(int) * kMaxBonds);
   L.cell_count = o; o = align256(o + sizeof(int) * kMaxCells);
   L.cell_start = o; o = align256(o + sizeof(int) * (kMaxCells + 1));
@@ -68,7 +67,6 @@ constexpr Layout make_layout() {
   L.e_cnt = o;      o = align256(o + sizeof(int) * kMaxBonds);
   L.scan_tmp = o;   o = align256(o + sizeof(int) * kScanTmp);
   L.bond_fil = o;   o = align256(o + sizeof(int) * kMaxBonds);
-  L.ub = o;         o = align256(o + sizeof(double) * 3 * kMaxBonds);
   L.g64 = o;        o = align256(o + sizeof(sc::BondGeomF64) * kMaxBonds);
   L.pa = o;         o = align256(o + sizeof(int) * kMaxPairs);
   L.pb = o;         o = align256(o + sizeof(int) * kMaxPairs);
@@ -77,8 +75,6 @@ constexpr Layout make_layout() {
   L.pf = o;         o = align256(o + sizeof(double) * 4 * kMaxPairs);
   L.cf = o;         o = align256(o + sizeof(double) * 16 * kMaxPairs);
   L.e_ent = o;      o = align256(o + sizeof(int) * 2 * kMaxPairs);
-  L.bF = o;         o = align256(o + sizeof(double) * 3 * kMaxBonds);
-  L.bT = o;         o = align256(o + sizeof(double) * 3 * kMaxBonds);
   L.status = o;     o = align256(o + sizeof(unsigned));
   L.counters = o;   o = align256(o + sizeof(unsigned long long) * 4);
   L.rep = o;        o = align256(o + sizeof(sc::ReplicaConst));

@@ -135,3 +135,37 @@ def test_noalloc_rejects_cell_grids_beyond_the_limit():
     f, t = _call_noalloc(system, fils, sites)
     assert np.array_equal(f, f_ref)
     assert np.array_equal(t, t_ref)
+
+
+# Filament bond counts, box side: one filament, two, two dimensions with equal
+# and uneven lengths, uneven ones in three; sizes that end a warp or a block.
+SHAPES = {
+    "one_3d": (3, [31], 30.0),
+    "one_short_2d": (2, [5], 12.0),
+    "two_2d": (2, [16, 16], 14.0),
+    "two_uneven_3d": (3, [5, 60], 40.0),
+    "equal_2d": (2, [16] * 32, 80.0),
+    "uneven_2d": (2, [5, 40, 9, 31, 32, 7, 100, 6, 66], 110.0),
+    "uneven_3d": (3, [5, 40, 9, 31, 32, 7, 100, 6, 26] * 3, 56.0),  # 49 cells a side of at most 50
+}
+
+
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_noalloc_shapes(name):
+    """Both dimensions, uneven offsets and the smallest sizes: the regular
+    entry points' forces, with interacting pairs (beside a single filament's own,
+    a copy of the first filament half a diameter away)."""
+    from test_gpu_team import _lattice
+    n_dim, n_seg, side = SHAPES[name]
+    system, fils, sites = _lattice(n_dim, np.array(n_seg), side, seed=7)
+    if len(n_seg) > 1:  # one more filament, beside the first
+        n = n_seg[0] + 1
+        system = dict(system)
+        fils = fils + [fils[0]]
+        sites = np.concatenate([sites, sites[:n] + np.array([0.3, 0.4, 0.0])])
+    f_ref, t_ref = _reference_forces(system, fils, sites)
+    assert np.abs(f_ref).max() > 0  # (one filament: bonds next but one)
+    for _ in range(2):
+        f, t = _call_noalloc(system, fils, sites)
+        assert np.array_equal(f, f_ref)
+        assert np.array_equal(t, t_ref)
