@@ -502,7 +502,7 @@ sc_status layout_integrator(sc_ctx *c) {
   int K = 1;
   std::vector<Bins> teams, teams2;
   const long long warps = pack_teams(1, teams);
-  if (warps > 148 * 20 && 4 * warps >= 9 * pack_teams(2, teams2)) {
+  if (warps > 20ll * c->n_sm && 4 * warps >= 9 * pack_teams(2, teams2)) {
     K = 2;
     teams.swap(teams2);
   }
@@ -854,6 +854,12 @@ sc_status sc_create(const sc_system_desc *desc, sc_ctx **out) {
           cudaSuccess) {
     cudaGetLastError();
     delete c;
+    return SC_ERR_CUDA;
+  }
+  if (cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, desc->device) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    sc_destroy(c);
     return SC_ERR_CUDA;
   }
   SysConst &k = c->k;

@@ -93,6 +93,7 @@ struct sc_ctx {
 
   // integrator blocks
   int nblocks = 0, C = 128;
+  int n_sm = 0;                    // the device's SMs
   int warp_sites = 32;             // longest filament for the team kernel
   int block_sites = 0;             // sites per block of the block kernel (0: 128, 256 or 512)
   int pair_block = 256;            // threads per block of the pair kernel (128 or 256)

@@ -277,3 +277,90 @@ def test_noise_precision_follows_the_system():
     assert np.array_equal(got[n:], alone[1])
     assert np.array_equal(got[:n], alone[0])
     both.close()
+
+
+def _two_a_lane(n_dim, side, seed, n=3100, extra=()):
+    """Mostly 17 to 20 sites, which fill a warp one filament at a time and
+    three at a time with two sites a lane; some short ones; `extra` bond counts.
+    More warps than 20 per SM, and 2.25 times those of the two-site layout."""
+    import torch
+    rng = np.random.default_rng(seed)
+    n_seg = np.concatenate([rng.choice([16, 17, 18, 19], n), [5, 8, 12] * 10, extra]).astype(int)
+    rng.shuffle(n_seg)
+    assert n > 20 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert n + 30 / 2 >= 2.25 * (n / 3 + 30 / 2 + 1)
+    return n_seg, _lattice(n_dim, n_seg, side, seed)
+
+
+def test_two_sites_a_lane_uneven_with_crosslinks_bitwise():
+    """Both integrator kernels, the table's lanes with two sites and one, and
+    tethers on the two bonds of a lane."""
+    import simcore_b200 as sc
+    from checkers import Oracle
+    n_seg, (system, fils, sites) = _two_a_lane(3, 330.0, 11, extra=[33, 45, 60] * 6)
+    first = np.concatenate([[0], np.cumsum(n_seg + 1)])
+    a = first[:400] + 3 + np.arange(400) % 3
+    b = first[1:401] + 2 + np.arange(400) % 4
+    ctx = sc.Context(system, fils, sites, precision="fp64")
+    oracle = Oracle(system, fils, sites)
+    for x in (ctx, oracle):
+        x.add_crosslinks(a, b, k_spring=0.05, rest_length=1.0)
+    for captured in (False, True):
+        (ctx.step_graph if captured else ctx.step)(4)
+        oracle.step(4)
+        assert np.array_equal(ctx.sites(), oracle.sites())
+        assert np.array_equal(ctx.crosslink_forces(), oracle.crosslink_forces())
+    assert np.abs(oracle.crosslink_forces()).max() > 0
+    ctx.close()
+    oracle.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_two_sites_a_lane_keep_systems_apart(precision):
+    """Two systems of one context in the two-site layout give the bits that
+    each gives alone, with one site a lane: fewer warps."""
+    import simcore_b200 as sc
+    parts = [_two_a_lane(2, 1400.0, 12)[1], _lattice(2, np.array([18, 16, 31, 7, 19]), 110.0, 13)]
+    fils = parts[0][1] + parts[1][1]
+    sites = np.concatenate([p[2] for p in parts])
+    replicas = [dict(system_radius=p[0]["system_radius"], seed=p[0]["seed"],
+                     n_filaments=len(p[1])) for p in parts]
+    both = sc.Context(parts[0][0], fils, sites, precision=precision, replicas=replicas)
+    both.step(3)
+    both.step_graph(4)
+    alone = []
+    for system, f, x in parts:
+        ctx = sc.Context(system, f, x, precision=precision)
+        ctx.step(3)
+        ctx.step_graph(4)
+        alone.append(ctx.sites())
+        ctx.close()
+    if precision == "fp64":
+        assert np.array_equal(both.sites(), np.concatenate(alone))
+    else:  # another elimination order: FP64 rounding, a few steps of it
+        n = len(alone[0])
+        assert np.array_equal(both.sites()[:n], alone[0])
+        assert np.abs(both.sites()[n:] - alone[1]).max() <= 1e-12 * 110.0
+    both.close()
+
+
+def test_two_sites_a_lane_fused_pairs():
+    """Fused pairs (every bond evaluates its own) against the split interface,
+    the lane's two bonds among them."""
+    import simcore_b200 as sc
+    system, fils, sites = _two_a_lane(2, 500.0, 14)[1]
+    a, b = (sc.Context(system, fils, sites, precision="mixed") for _ in range(2))
+    for c in (a, b):
+        c.set_exact_near_parallel(False)
+    a.set_fused_pairs(True)
+    a.step(3)
+    a.step_graph(6)
+    for _ in range(9):
+        b.interact()
+        b.update_positions()
+    assert len(b.pairs()) > 1000
+    assert np.array_equal(a.sites(), b.sites())
+    for x, y in zip(a.bond_forces(), b.bond_forces()):
+        assert np.array_equal(x, y)
+    a.close()
+    b.close()
