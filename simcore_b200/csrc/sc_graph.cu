@@ -13,8 +13,17 @@ using namespace scapi;
 // 31.8, 16,000 bonds the same; beyond, one cluster's rebuild (125 us at 20,000
 // bonds) costs more than the loop's conditional nodes.  The cluster also scans
 // one counter per 32 cells; the suspensions of these sizes have up to 11,000.
+// A rebuild's candidate pairs cost the cluster about 3 ns each more than the
+// rebuild's own kernels, so dense lists take the graph: 12,000 bonds with 8,000
+// pairs 28.7 us chained, 31.1 in the graph (mixed), with 34,000 44.1 and 42.8,
+// with 160,000 in a buckling network, rebuilt every step, 777 and 334; 2,000
+// bonds with 9,300 pairs 44.0 and 48.1, with 23,500 rebuilt every step 293 and
+// 259; 300 bonds with 3,600, rebuilt every step, 213 and 202.  64 systems of
+// 12,200 bonds and 5,000 pairs, rebuilt every step: 59.9 and 63.5.
 static const int kChainBonds = 12288;
 static const int kChainGroups = 32768;
+static const int kChainPairs = 16384;
+static const int kChainPairsPerBond = 6;
 // BD steps queued at a time: what a run that stops early still launches for
 // nothing (about 2 us a launch), against a synchronisation and an empty queue
 // (about 15 us) per 9 ms or more of steps.
@@ -138,10 +147,12 @@ static sc_status build_graph(sc_ctx *c) {
   return SC_OK;
 }
 
-// Whether a captured run is launched as a chain.
+// Whether a captured run, whose pair count is known, is launched as a chain.
 static bool chained(const sc_ctx *c) {
   if (!c->desc.interaction_flag || c->run_form == SC_RUN_GRAPH) return false;
-  return c->run_form == SC_RUN_CHAIN || (c->nb <= kChainBonds && c->rb.n_groups <= kChainGroups);
+  return c->run_form == SC_RUN_CHAIN ||
+         (c->nb <= kChainBonds && c->rb.n_groups <= kChainGroups && c->np <= kChainPairs &&
+          c->np <= (long long)kChainPairsPerBond * c->nb);
 }
 
 sc_status sc_set_run_form(sc_ctx *c, sc_run_form form) {

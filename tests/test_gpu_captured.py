@@ -203,3 +203,27 @@ def test_long_chain_is_queued_in_pieces():
         ctx.step_graph(4000)
     assert e.value.code == 7
     assert ctx.counters().kernel_launches - before <= 512 * 5 + 3
+
+
+@pytest.mark.parametrize("side,form", [(80.0, "chain"), (16.0, "graph")])
+def test_default_form_by_pairs(side, form):
+    """A sparse small system takes the chain, a dense one (more than six pairs
+    a bond) the graph: a run with rebuilds makes as many launches as that form
+    (a rebuild's kernels are launches in the graph alone)."""
+    from test_gpu_team import _lattice
+    n_fil = 144
+    system, fils, sites = _lattice(2, np.array([10] * n_fil), side, seed=3)
+    system = dict(system, delta=1e-5, wca_eps=0.01)
+    made = {}
+    for f in ("auto", "graph", "chain"):
+        ctx = _ctx(system, fils, sites, "mixed")
+        ctx.set_run_form(f)
+        n_pairs = ctx.counters().n_pairs
+        before = ctx.counters()
+        ctx.step_graph(3000)
+        after = ctx.counters()
+        assert after.n_rebuilds > before.n_rebuilds
+        made[f] = after.kernel_launches - before.kernel_launches
+    assert (n_pairs > 6 * 10 * n_fil) == (form == "graph")
+    assert made["graph"] != made["chain"]
+    assert made["auto"] == made[form]
