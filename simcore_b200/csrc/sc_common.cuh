@@ -155,6 +155,11 @@ struct DevState {
   // filament, its index | filament sites << 16, its filament in the block.
   const int2 *blk_list;
   const int4 *blk_slot;
+  // Static crosslinks (the xl_ and xb_ arrays).  (Here and not beside them for the
+  // offsets of the arrays between in the kernels' constants: with r and ub 8 bytes
+  // lower the analyses' two kernels took 123 us on 20,000 bonds, 119 so; every
+  // other case measured the same.)
+  int nx;
   // Equal filaments of blk_uni_n sites, blk_uni_fpb to a block, every block
   // but the last full, sites numbered filament by filament from 0: blocks
   // and sites then find their filaments by arithmetic (0: read the tables).
@@ -197,8 +202,7 @@ struct DevState {
   long long *th_nrec;      // per system: records written
   double *th_rec;          // ring of th_cap records per system: i_step, tensor (9), pressure, volume
   int th_cap, th_gx, th_n;
-  // static crosslinks (harmonic tethers between two bonds)
-  int nx;                  // links
+  // static crosslinks (nx harmonic tethers between two bonds)
   const int *xl_fil;       // 2 per link: filament of each anchor
   double *xl_M;            // 2 per link: mesh lambda of each anchor (Anchor::mesh_lambda_)
   double *xl_c;            // 8 per anchor: force (3), torque (3), its bond, pad

@@ -506,7 +506,7 @@ __global__ void k_rb_csr_sort(DevState d, RebuildBufs rb) {
 // launched one after another, and one cluster of blocks between them ends a
 // step, decides the next one's rebuild and does it when due, phase by phase
 // over the hardware's cluster barrier (the kernels above, over all items in
-// turn).  2,000 bonds, 10 BD steps: 320 us with the loop, 256 so.  Idle it is
+// turn).  2,000 bonds, 10 BD steps: 320 us with the loop, 270 so.  Idle it is
 // bound by its launch and three dependent round trips to L2 (4 us); a rebuild
 // by the phases' latencies, 36 us at 2,000 bonds (as the ten kernels), 125 at
 // 20,000.  A cluster and not the chip: its barrier needs no waiting loop and
