@@ -530,7 +530,7 @@ def run_ours(args, rank, world, local_rank):
         "data": "synthetic (seeded random insertion with overlap rejection)",
         "config": workload_config(args.workload),
         "run": {"precision": "mixed", "i_steps_per_step": I_STEPS_PER_STEP,
-                "timed_unit": "one CUDA-graph launch of 20 reference steps (WHILE loop of 10 "
+                "timed_unit": "one captured run of 20 reference steps (sc_step_graph: 10 "
                               "midpoint BD steps with device-decided pair-list rebuilds)",
                 "l2": "flushed by a 256 MiB write before every timed step",
                 "parallelism": ("independent systems shared out over %d ranks" % world
