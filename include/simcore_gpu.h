@@ -276,7 +276,9 @@ sc_status sc_step_graph(sc_ctx *ctx, int n);
 /* The form of sc_step_graph's runs: SC_RUN_AUTO (default) picks by the system's
  * size, SC_RUN_GRAPH always replays the captured graph, SC_RUN_CHAIN always
  * launches the steps one after another (systems without interactions have the
- * graph alone).  Every form gives the same results. */
+ * graph alone).  Every form gives the same results.  A chain's launches are
+ * host work: a program that steps a dozen or more small contexts at once, each
+ * from its own thread, may find the graph faster. */
 typedef enum { SC_RUN_AUTO = 0, SC_RUN_GRAPH = 1, SC_RUN_CHAIN = 2 } sc_run_form;
 sc_status sc_set_run_form(sc_ctx *ctx, sc_run_form form);
 /* Waits for the context's stream and reports any deferred device error. */
