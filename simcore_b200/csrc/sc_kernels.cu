@@ -689,7 +689,7 @@ __device__ __forceinline__ void near_parallel_fp64(const SysConst &k, const DevS
 // evaluates nothing: the forces stay the last step's, however many launches the
 // chain still holds.  (The halting bits are the rebuild's and the control
 // kernel's: as old as the list.  A graph holds none past the step that stops it,
-// and the load costs several systems' larger lists 0.4 us a launch.)
+// and a test among its loads costs several systems' larger lists 0.4 us a launch.)
 // NPX (mixed only): nearly parallel pairs are evaluated in FP64
 // (eval_near_parallel) by the thread that meets them.
 // The list and its slot indices date from the last rebuild, whose kernels
@@ -701,11 +701,13 @@ template <int ND, int PREC, bool NPX, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
     k_pair_eval(SysConst k, DevState d, int rbuf, int wait_first, int chained) {
   if (wait_first) grid_dep_sync();
-  const bool halted = chained && (*d.status & ST_HALT) != 0u;
+  if (chained && (*d.status & ST_HALT)) {
+    if (!wait_first) grid_dep_sync();  // whoever waits for this kernel has waited for all
+    return;
+  }
   if (d.nrep == 1) {
     const ReplicaConst &R = d.rep[0];
-    const int listed = d.np_rep[0];
-    const int np = halted | (listed > R.pcap) ? 0 : listed;  // (no branch: the loads are one trip)
+    const int np = d.np_rep[0] <= R.pcap ? d.np_rep[0] : 0;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     PairIdx ix = {0, 0, 0, 0};
     if (p < np) ix = pair_idx(d, p);
@@ -727,7 +729,7 @@ __global__ void __launch_bounds__(BLOCK, NPX ? 1024 / BLOCK : 1)
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < d.pcap_total;
        p += gridDim.x * blockDim.x) {
     int r;
-    if (pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap && !halted &&
+    if (pair_live(d, p, r) && d.np_rep[r] <= d.rep[r].pcap &&
         !pair_eval_one<ND, PREC, NPX>(k, d, d.rep[r], rbuf, p, pair_idx(d, p)))
       if (NPX) near_parallel_fp64<ND>(k, d, d.rep[r], p);
   }
